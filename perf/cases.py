@@ -296,18 +296,18 @@ def prepare(case, seed):
         return dict(case=case, net=net, a=a, target=target)
     if kind == "sweep":
         from polarism_gb300.engine import MemberPhysics
-        from polarism_gb300.sweep import SweepEngine
+        from polarism_gb300.sweep import SweepEngine, autotune_tiling
 
         x = _sweep_inputs(case, seed)
         members = len(x["sizes"])
         eng = SweepEngine([(n, n, 0.5, 0.5) for n in x["sizes"]], [MemberPhysics(**PHYSICS)] * members,
                           case["dt"])
-        eng.set_tiling(512, 64)
         eng.set_pump([e.cpu().numpy() for e in x["envs"]])
         if case["noise"]:
             ones = np.ones(members)
             eng.set_noise(x["seeds"], PHYSICS["gamma_C"] * ones, PHYSICS["R"] * ones, ones)
         torch.cuda.synchronize()
+        autotune_tiling(eng, noise=case["noise"], use_cache=False)  # as a sweep run does before its steps
         return dict(case=case, eng=eng, psi=x["psi"], res=x["res"], psi_out=torch.empty_like(x["psi"]),
                     res_out=torch.empty_like(x["res"]), scales=np.full((case["steps"], 3, members), P0))
     if kind == "dropin":
