@@ -196,6 +196,14 @@ bool use_quad(const pg_solver* s, const pg::WideGeom& w) {
          pg::quad_rk4_supported(s->cfg.nx, s->cfg.ny);
 }
 
+// The tile kernel steps every FP64 grid unless the caller chose the streaming kernel or its
+// geometry: measured without / with Wigner noise, us a step, streaming kernel -> tile kernel:
+// 92.6 -> 11.4 / 141 -> 14.7 at 128^2, 179 -> 24.4 / 269 -> 35.9 at 256^2, 208 -> 78 / 314 -> 123
+// at 512^2, 310 -> 268 / 495 -> 426 at 1024^2.
+bool use_tile(const pg_solver* s) {
+  return s->rk4_kernel != 1 && !s->geom_set && s->cfg.precision == PG_DOUBLE;
+}
+
 // Launch one RK4 step reading buffers of parity `from`; step_offset indexes the chunk scales.
 cudaError_t launch_step(pg_solver* s, int from, int step_offset) {
   const int to = 1 - from;
@@ -238,6 +246,13 @@ cudaError_t launch_step(pg_solver* s, int from, int step_offset) {
   g.pot_stride = s->cfg.potential_per_member ? s->plane : 0;
   g.halt = s->halt;
   g.pump_term_stride = s->pump_term_stride;
+  if (use_tile(s))
+    return pg::launch_rk4_tile_f64(
+        s->tile_shape, static_cast<const double*>(s->psi[from]), static_cast<const double*>(s->res[from]),
+        static_cast<const double*>(s->pump), static_cast<const double*>(s->potential),
+        static_cast<double*>(s->psi[to]), static_cast<double*>(s->res[to]),
+        static_cast<const pg::RhsConst<double>*>(s->consts), static_cast<const double*>(s->scales),
+        s->step_base, step_offset, s->cfg.dt, s->noise, g, f, s->stream);
   if (s->cfg.precision == PG_DOUBLE) {
     return pg::launch_rk4_step<double>(
         static_cast<const double*>(s->psi[from]), static_cast<const double*>(s->res[from]),
@@ -425,6 +440,8 @@ int pg_create(const pg_config* cfg, const pg_physics* physics, pg_solver** out) 
       return fail(e, "staging event");
   }
   pg::choose_rk4_geometry(cfg->nx, cfg->ny, cfg->members, cfg->precision, s->sm_count, &s->geom);
+  if (cfg->precision == PG_DOUBLE)
+    s->tile_shape = pg::choose_rk4_tile_f64(cfg->nx, cfg->ny, cfg->members, s->sm_count);
   int rc = upload_consts(s);
   if (rc != PG_OK) {
     release(s);
@@ -637,6 +654,7 @@ int pg_rk4_set_geometry(pg_solver* s, int32_t tile_w, int32_t strip_h) {
     s->geom.tile_w = tile_w;
   }
   s->geom.strip_h = strip_h;
+  s->geom_set = true;
   free_graphs(s);
   return PG_OK;
 }

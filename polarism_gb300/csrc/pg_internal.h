@@ -95,6 +95,16 @@ cudaError_t launch_rk4_step(const T* psi_in, const T* n_in, const T* pump, const
                             int step_offset, T dt, bool noise, const RK4Geom& g,
                             const RK4Features& f, cudaStream_t stream);
 
+// The same step on two-dimensional tiles (rk4_tile.cuh), bit for bit; `shape` indexes the tile
+// shapes, choose_rk4_tile_f64 picks one for a grid.
+int choose_rk4_tile_f64(int nx, int ny, int members, int sm_count);
+cudaError_t launch_rk4_tile_f64(int shape, const double* psi_in, const double* n_in, const double* pump,
+                                const double* potential, double* psi_out, double* n_out,
+                                const RhsConst<double>* consts, const double* scales,
+                                const unsigned long long* step_base, int step_offset, double dt,
+                                bool noise, const RK4Geom& g, const RK4Features& f,
+                                cudaStream_t stream);
+
 // Choose the tile width / strip height for a grid (deterministic heuristic,
 // overridable through the autotuner table).
 void choose_rk4_geometry(int nx, int ny, int members, int precision, int sm_count,

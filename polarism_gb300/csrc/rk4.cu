@@ -19,23 +19,10 @@
 // write of psi and n per site (28 B/site in FP32) plus the strip/tile halos.
 #include "philox.cuh"
 #include "pg_internal.h"
+#include "rk4_general.cuh"
 
 namespace pg {
 namespace {
-
-template <typename T>
-struct Cplx;
-template <>
-struct Cplx<float> {
-  using type = float2;
-};
-template <>
-struct Cplx<double> {
-  using type = double2;
-};
-
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
 template <typename T>
 struct MaxThreads;
@@ -47,53 +34,6 @@ template <>
 struct MaxThreads<double> {
   static constexpr int value = 288;
 };
-
-// One right-hand-side evaluation at a site.  c is the centre, (lt, rt, up, dn) the
-// four neighbours, n the active reservoir density, sP the scaled pump.
-// n2 is the inactive reservoir of the two-field reservoirs (double: n_I feeding n_A,
-// polarism/reservoir/double_reservoir.py:106-130; quadratic-double: n_I feeding n_R through
-// kappa n_I^2, quadratic_double_reservoir.py:13-14); dn2 its derivative.
-template <typename T, bool GENERAL, bool TWO>
-__device__ __forceinline__ void site_rhs(const typename Cplx<T>::type c,
-                                         const typename Cplx<T>::type lt,
-                                         const typename Cplx<T>::type rt,
-                                         const typename Cplx<T>::type up,
-                                         const typename Cplx<T>::type dn, const T n, const T sP,
-                                         const RhsConst<T>& k, const T vre, const T vim,
-                                         const RK4Features& f, T& dre, T& dim, T& dnr,
-                                         const T n2, T& dn2) {
-  const T rho = c.x * c.x + c.y * c.y;
-  const T lre = k.ax * (lt.x + rt.x) + k.ay * (up.x + dn.x);
-  const T lim = k.ax * (lt.y + rt.y) + k.ay * (up.y + dn.y);
-  T w = k.w0 + k.gc * rho + k.gr * n;
-  T gl = k.half_R * n - k.half_gC;
-  if (GENERAL) {
-    w += vre * k.inv_hbar;
-    gl += vim * k.inv_hbar;
-    if (TWO) w += k.gi * n2;
-  }
-  dre = gl * c.x + w * c.y - lim;
-  dim = gl * c.y - w * c.x + lre;
-  if (GENERAL && f.relax) {
-    const T en = k.eta_a * n;
-    dre += en * (lre - k.w0 * c.x);
-    dim += en * (lim - k.w0 * c.y);
-  }
-  dnr = sP - (k.gamma_R + k.R * rho) * n;
-  dn2 = T(0);
-  if (GENERAL) {
-    if (f.reservoir == 0) {
-      dnr = T(0);
-    } else if (TWO && f.reservoir == 2) {
-      dn2 = sP - (k.gamma_I + k.R_IA) * n2 + k.R_AI * n;
-      dnr = k.R_IA * n2 - (k.gamma_A + k.R_AI + k.R * rho) * n;
-    } else if (TWO && f.reservoir == 3) {
-      const T transfer = k.kappa * n2 * n2;
-      dnr = transfer - k.gamma_R * n - k.R * n * rho;
-      dn2 = sP - transfer - k.gamma_I * n2;
-    }
-  }
-}
 
 template <typename T, bool NOISE, bool GENERAL, bool TWO>
 __global__ void __launch_bounds__(MaxThreads<T>::value, 1)
@@ -244,19 +184,20 @@ __global__ void __launch_bounds__(MaxThreads<T>::value, 1)
           vre = f.potential == 2 ? pot_m[2 * o] : pot_m[o];
           vim = f.potential == 2 ? pot_m[2 * o + 1] : T(0);
         }
-        T dre, dim, dnr, du;
+        C2 d;
+        T dnr, du;
         const T sP = multi ? pump_terms_value(pump_m, g.pump_term_stride, c0, m_count, L,
                                               static_cast<long long>(ra) * nx + gx)
-                           : mul_rn(s0, P[sa]);
-        site_rhs<T, GENERAL, TWO>(p0[sa], xin[lt_i], xin[rt_i], p0[sb], p0[j], n0[sa],
-                             sP, k, vre, vim, f, dre, dim, dnr, u0[sa], du);
-        q1[sa] = C2{p0[sa].x + hh * dre, p0[sa].y + hh * dim};
-        m1[sa] = n0[sa] + hh * dnr;
-        acc[sa] = C2{p0[sa].x + h6 * dre, p0[sa].y + h6 * dim};
-        accn[sa] = n0[sa] + h6 * dnr;
+                           : pump_mul_rn(s0, P[sa]);
+        general_rhs<T, GENERAL, TWO>(p0[sa], xin[lt_i], xin[rt_i], p0[sb], p0[j], n0[sa],
+                             sP, k, vre, vim, f, d, dnr, u0[sa], du);
+        q1[sa] = axpy_t<T>(hh, d, p0[sa]);
+        m1[sa] = fma_t(hh, dnr, n0[sa]);
+        acc[sa] = axpy_t<T>(h6, d, p0[sa]);
+        accn[sa] = fma_t(h6, dnr, n0[sa]);
         if (two) {
-          v1[sa] = u0[sa] + hh * du;
-          accu[sa] = u0[sa] + h6 * du;
+          v1[sa] = fma_t(hh, du, u0[sa]);
+          accu[sa] = fma_t(h6, du, u0[sa]);
         }
       }
       // Stage 2 at row r-2: k2 = f(psi1).
@@ -268,24 +209,25 @@ __global__ void __launch_bounds__(MaxThreads<T>::value, 1)
           vre = f.potential == 2 ? pot_m[2 * o] : pot_m[o];
           vim = f.potential == 2 ? pot_m[2 * o + 1] : T(0);
         }
-        T dre, dim, dnr, du;
+        C2 d;
+        T dnr, du;
         const C2* xr = xin + nthreads;
-        T sP = mul_rn(s1, P[sb]);
+        T sP = pump_mul_rn(s1, P[sb]);
         if (multi) {
           int rb = row_load - 2;
           if (rb < 0) rb += ny;
           sP = pump_terms_value(pump_m, g.pump_term_stride, c1, m_count, L,
                                 static_cast<long long>(rb) * nx + gx);
         }
-        site_rhs<T, GENERAL, TWO>(q1[sb], xr[lt_i], xr[rt_i], q1[sc], q1[sa], m1[sb],
-                             sP, k, vre, vim, f, dre, dim, dnr, v1[sb], du);
-        q2[sb] = C2{p0[sb].x + hh * dre, p0[sb].y + hh * dim};
-        m2[sb] = n0[sb] + hh * dnr;
-        acc[sb] = C2{acc[sb].x + h3 * dre, acc[sb].y + h3 * dim};
-        accn[sb] = accn[sb] + h3 * dnr;
+        general_rhs<T, GENERAL, TWO>(q1[sb], xr[lt_i], xr[rt_i], q1[sc], q1[sa], m1[sb],
+                             sP, k, vre, vim, f, d, dnr, v1[sb], du);
+        q2[sb] = axpy_t<T>(hh, d, p0[sb]);
+        m2[sb] = fma_t(hh, dnr, n0[sb]);
+        acc[sb] = axpy_t<T>(h3, d, acc[sb]);
+        accn[sb] = fma_t(h3, dnr, accn[sb]);
         if (two) {
-          v2[sb] = u0[sb] + hh * du;
-          accu[sb] = accu[sb] + h3 * du;
+          v2[sb] = fma_t(hh, du, u0[sb]);
+          accu[sb] = fma_t(h3, du, accu[sb]);
         }
       }
       // Stage 3 at row r-3: k3 = f(psi2).
@@ -297,24 +239,25 @@ __global__ void __launch_bounds__(MaxThreads<T>::value, 1)
           vre = f.potential == 2 ? pot_m[2 * o] : pot_m[o];
           vim = f.potential == 2 ? pot_m[2 * o + 1] : T(0);
         }
-        T dre, dim, dnr, du;
+        C2 d;
+        T dnr, du;
         const C2* xr = xin + 2 * nthreads;
-        T sP = mul_rn(s1, P[sc]);
+        T sP = pump_mul_rn(s1, P[sc]);
         if (multi) {
           int rc = row_load - 3;
           if (rc < 0) rc += ny;
           sP = pump_terms_value(pump_m, g.pump_term_stride, c1, m_count, L,
                                 static_cast<long long>(rc) * nx + gx);
         }
-        site_rhs<T, GENERAL, TWO>(q2[sc], xr[lt_i], xr[rt_i], q2[sd], q2[sb], m2[sc],
-                             sP, k, vre, vim, f, dre, dim, dnr, v2[sc], du);
-        q3[sc] = C2{p0[sc].x + dt * dre, p0[sc].y + dt * dim};
-        m3[sc] = n0[sc] + dt * dnr;
-        acc[sc] = C2{acc[sc].x + h3 * dre, acc[sc].y + h3 * dim};
-        accn[sc] = accn[sc] + h3 * dnr;
+        general_rhs<T, GENERAL, TWO>(q2[sc], xr[lt_i], xr[rt_i], q2[sd], q2[sb], m2[sc],
+                             sP, k, vre, vim, f, d, dnr, v2[sc], du);
+        q3[sc] = axpy_t<T>(dt, d, p0[sc]);
+        m3[sc] = fma_t(dt, dnr, n0[sc]);
+        acc[sc] = axpy_t<T>(h3, d, acc[sc]);
+        accn[sc] = fma_t(h3, dnr, accn[sc]);
         if (two) {
-          v3[sc] = u0[sc] + dt * du;
-          accu[sc] = accu[sc] + h3 * du;
+          v3[sc] = fma_t(dt, du, u0[sc]);
+          accu[sc] = fma_t(h3, du, accu[sc]);
         }
       }
       // Stage 4 at row r-4: k4 = f(psi3), final combine, clamp, Wigner increment.
@@ -324,23 +267,24 @@ __global__ void __launch_bounds__(MaxThreads<T>::value, 1)
           vre = f.potential == 2 ? pot_m[2 * o] : pot_m[o];
           vim = f.potential == 2 ? pot_m[2 * o + 1] : T(0);
         }
-        T dre, dim, dnr, du;
+        C2 d;
+        T dnr, du;
         const C2* xr = xin + 3 * nthreads;
         const T sP = multi ? pump_terms_value(pump_m, g.pump_term_stride, c2, m_count, L,
                                               static_cast<long long>(row_out) * nx + gx)
-                           : mul_rn(s2, P[sd]);
-        site_rhs<T, GENERAL, TWO>(q3[sd], xr[lt_i], xr[rt_i], q3[sa], q3[sc], m3[sd],
-                             sP, k, vre, vim, f, dre, dim, dnr, v3[sd], du);
-        T ore = acc[sd].x + h6 * dre;
-        T oim = acc[sd].y + h6 * dim;
-        T on = accn[sd] + h6 * dnr;
+                           : pump_mul_rn(s2, P[sd]);
+        general_rhs<T, GENERAL, TWO>(q3[sd], xr[lt_i], xr[rt_i], q3[sa], q3[sc], m3[sd],
+                             sP, k, vre, vim, f, d, dnr, v3[sd], du);
+        T ore = fma_t(h6, d.x, acc[sd].x);
+        T oim = fma_t(h6, d.y, acc[sd].y);
+        T on = fma_t(h6, dnr, accn[sd]);
         on = on < T(0) ? T(0) : on;
-        T ou = two ? accu[sd] + h6 * du : T(0);
+        T ou = two ? fma_t(h6, du, accu[sd]) : T(0);
         ou = ou < T(0) ? T(0) : ou;
         if (i >= 8 && i - 8 < h_eff && col_writes) {
           const long long o = static_cast<long long>(row_out) * nx + gx;
           if (NOISE) {
-            WignerDraw<T>::apply(wz, k.noise_a + k.noise_b * on, ore, oim);
+            WignerDraw<T>::apply(wz, fma_t(k.noise_b, on, k.noise_a), ore, oim);
           }
           psi_out[member * plane + o] = C2{ore, oim};
           if (!GENERAL || f.reservoir) n_out[member * plane + o] = on;

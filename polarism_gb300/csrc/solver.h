@@ -41,6 +41,8 @@ struct pg_solver {
   std::vector<double> noise_gamma, noise_R, noise_strength;
   double dt_over_4dv = 0.0;
   pg::RK4Geom geom{};
+  bool geom_set = false;     // pg_rk4_set_geometry chose it: the streaming kernel runs with it
+  int tile_shape = 0;        // tile of the tile kernel (choose_rk4_tile_f64)
   // Pinned staging ring for chunk scales and the step base.
   struct Slot {
     void* host = nullptr;
