@@ -98,6 +98,29 @@ int setup_tables(pg_solver* s) {
   PG_CUDA(cudaMemcpyAsync(s->prop, prop.data(), prop.size() * sizeof(T), cudaMemcpyHostToDevice,
                           s->stream));
   PG_CUDA(configure_split_kernels<T>(200 * 1024));
+  // Tables of the register-resident passes.
+  std::vector<T> reg_host[2];
+  for (int axis = 0; axis < 2; ++axis) {
+    const int n = axis == 0 ? nx : ny;
+    if (sizeof(T) == 8 || !reg_fft_size(n)) continue;
+    const int vals = reg_fft_vals(n), M = n / vals;
+    std::vector<T>& tab = reg_host[axis];
+    tab.resize(static_cast<size_t>(4) * n);
+    for (int k = 0; k < vals; ++k)
+      for (int t = 0; t < M; ++t) {
+        const double ang = -2.0 * kPi * static_cast<double>(t * k) / n;
+        const double cr = std::cos(ang), ci = std::sin(ang);
+        T* o = tab.data() + static_cast<size_t>(4) * (k * M + t);
+        o[0] = static_cast<T>(cr);
+        o[1] = static_cast<T>(ci);
+        o[2] = static_cast<T>(cr - static_cast<double>(o[0]));
+        o[3] = static_cast<T>(ci - static_cast<double>(o[1]));
+      }
+    void*& dst = axis == 0 ? s->reg_x : s->reg_y;
+    PG_CUDA(cudaMalloc(&dst, tab.size() * sizeof(T)));
+    PG_CUDA(cudaMemcpyAsync(dst, tab.data(), tab.size() * sizeof(T), cudaMemcpyHostToDevice, s->stream));
+  }
+  if (s->reg_x != nullptr || s->reg_y != nullptr) PG_CUDA(configure_split_reg(nx, ny));
   if (sizeof(T) == 4 && (split_fast_row(nx, ny) || split_fast_col(nx, ny))) {
     std::vector<float> tw4(4 * 1024);
     split_fast_twiddles(tw4.data());
@@ -177,8 +200,14 @@ PassPlan plan(const pg_solver* s) {
   r.nx = c.nx;
   r.ny = c.ny;
   r.log2nx = ilog2(c.nx);
+  // Whole rows up to 4096 sites a block, but at least two blocks an SM where the grid has them: a
+  // 256^2 double-precision grid otherwise runs its row passes on 16 SMs (92 us a pass; the FP64
+  // pipe bounds it, so its time is that of the busiest SM).
+  const long long want_blocks = 2LL * std::max(1, s->sm_count);
   int rows = 1;
-  while (rows * 2 <= c.ny && rows * 2 * c.nx <= 4096) rows *= 2;
+  while (rows * 2 <= c.ny && rows * 2 * c.nx <= 4096 &&
+         static_cast<long long>(c.ny / (rows * 2)) * c.members >= want_blocks)
+    rows *= 2;
   r.rows = rows;
   r.log2rows = ilog2(rows);
   // mv values a thread, or down to four when the grid would not fill the GPU otherwise.
@@ -200,9 +229,12 @@ PassPlan plan(const pg_solver* s) {
   // an SM and one block's loads and stores overlap another's transforms.  At 1024^2 this ran
   // 10% faster than sixteen-column blocks of 1024 threads (one block per SM); two columns
   // (half a DRAM sector a row) ran 30% slower.
+  // Fewer (down to one sector's columns) where a small grid would not give two blocks an SM.
+  const int min_cols = static_cast<int>(std::min<size_t>(static_cast<size_t>(c.nx), 32 / csize));
   int cols = 1;
   while (cols * 2 <= c.nx && cols * 2 <= 4 && cols * 2 * c.ny * csize <= 160 * 1024 &&
-         cols * 2 * c.ny <= mv * 1024)
+         cols * 2 * c.ny <= mv * 1024 &&
+         (cols < min_cols || static_cast<long long>(c.nx / (cols * 2)) * c.members >= want_blocks))
     cols *= 2;
   k.cols = cols;
   k.log2cols = ilog2(cols);
@@ -237,10 +269,10 @@ cudaError_t row_launch(pg_solver* s, const PassPlan& p, int forward, int table, 
                 (static_cast<size_t>(table < 0 ? 0 : table) * s->cfg.members * per) * 2;
   const T* py = px + static_cast<size_t>(s->cfg.nx) * 2;
   // Member m's factors start at px + m * (nx + ny) complex values (py follows its px).
-  if (sizeof(T) == 4 && s->tw4 != nullptr && split_fast_row(s->cfg.nx, s->cfg.ny))
-    return launch_row_fast(static_cast<float*>(s->psi[s->cur]), static_cast<const float*>(s->tw4),
-                           reinterpret_cast<const float*>(px), reinterpret_cast<const float*>(py),
-                           a, s->cfg.members, s->stream);
+  if (s->reg_x != nullptr)
+    return launch_row_reg(static_cast<float*>(s->psi[s->cur]), static_cast<const float*>(s->reg_x),
+                          reinterpret_cast<const float*>(px), reinterpret_cast<const float*>(py), a,
+                          s->cfg.members, s->sm_count, s->stream);
   return launch_row_pass<T>(static_cast<T*>(s->psi[s->cur]), static_cast<const T*>(s->tw_x), px,
                             py, a, s->cfg.members, s->stream);
 }
@@ -254,12 +286,13 @@ cudaError_t col_launch(pg_solver* s, const PassPlan& p, int inverse, int op, int
   a.op = op;
   a.scale_offset = scale_offset;
   a.step_offset = step_offset;
-  if (sizeof(T) == 4 && s->tw4 != nullptr && split_fast_col(s->cfg.nx, s->cfg.ny))
-    return launch_col_fast(static_cast<float*>(s->psi[s->cur]), static_cast<float*>(s->res[s->cur]),
-                           static_cast<const float*>(s->pump), static_cast<const float*>(s->potential),
-                           static_cast<const float*>(s->tw4),
-                           static_cast<const SplitConst<float>*>(s->split_consts),
-                           static_cast<const float*>(s->scales), s->step_base, a, s->stream);
+  if (s->reg_y != nullptr)
+    return launch_col_reg(static_cast<float*>(s->psi[s->cur]), static_cast<float*>(s->res[s->cur]),
+                          static_cast<const float*>(s->pump), static_cast<const float*>(s->potential),
+                          static_cast<const float*>(s->reg_y),
+                          static_cast<const SplitConst<float>*>(s->split_consts),
+                          static_cast<const float*>(s->scales), s->step_base, a,
+                          s->sm_count, s->stream);
   return launch_col_pass<T>(static_cast<T*>(s->psi[s->cur]), static_cast<T*>(s->res[s->cur]),
                             static_cast<const T*>(s->pump), static_cast<const T*>(s->potential),
                             static_cast<const T*>(s->tw_y),
@@ -402,6 +435,9 @@ int split_release(pg_solver* s) {
   cudaFree(s->tw_y);
   cudaFree(s->tw4);
   s->tw4 = nullptr;
+  cudaFree(s->reg_x);
+  cudaFree(s->reg_y);
+  s->reg_x = s->reg_y = nullptr;
   cudaFree(s->prop);
   cudaFree(s->split_consts);
   s->tw_x = s->tw_y = s->prop = s->split_consts = nullptr;

@@ -1,0 +1,88 @@
+// Launch shapes and synchronisation shared by the register-resident row and column passes
+// (split_reg.cuh, ifrk_reg.cuh).
+#pragma once
+#include <algorithm>
+
+#include "fft_reg.cuh"
+
+namespace pg {
+namespace {
+
+// Barrier over the threads of one transform (or of a row's transforms): within a warp, or a named
+// barrier of `count` threads.
+template <bool WARP>
+struct GroupSync {
+  int id, count;
+  __device__ __forceinline__ void operator()() const {
+    if constexpr (WARP)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+  }
+};
+struct BlockSync {
+  __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+
+// Row pass: `rows` rows of COMPS components a block, N / V threads each.  Rows of fewer than 16
+// threads share half-warps: their buffers are offset so that the half-warp's accesses stay on
+// distinct banks.
+template <int N, int V, int COMPS>
+struct RowShape {
+  static constexpr int M = RegFft<N, V>::M;
+  static constexpr int GROUP = M * COMPS;  // threads of one row
+  static constexpr int STRIDE = RegFft<N, V>::SLOTS + (M < 16 ? M : 0);
+  static constexpr int MAX_THREADS = GROUP > 256 ? GROUP : 256;
+};
+
+// Rows a block: 256 threads, fewer (down to a warp, or one row) where the grid would not give two
+// blocks an SM.
+template <int N, int V, int COMPS>
+int row_shape_rows(int ny, int members, int sm_count) {
+  using S = RowShape<N, V, COMPS>;
+  int rows = std::max(1, std::min(ny, 256 / S::GROUP));
+  while (rows > 1 && rows / 2 * S::GROUP >= 32 &&
+         static_cast<long long>(ny / rows) * members < 2LL * sm_count)
+    rows /= 2;
+  return rows;
+}
+
+// Column pass: `cols` columns of COMPS components a block.
+template <typename T, int N, int V, int COMPS>
+struct ColShape {
+  static constexpr int M = RegFft<N, V>::M;
+  static constexpr int SLOTS = RegFft<N, V>::SLOTS;
+  static constexpr int REGS = sizeof(T) == 4 ? 64 : 128;  // a thread
+  static constexpr int LIMIT = sizeof(T) == 4 ? 1024 : 512;
+  // 64-byte row segments (8 FP32 columns, 4 FP64), fewer where the block would be too large.
+  static constexpr int WANT = sizeof(T) == 4 ? 8 : 4;
+  static constexpr int cap(int want, int limit) {
+    int c = want;
+    while (c > 1 && c * M * COMPS > limit) c /= 2;
+    return c;
+  }
+  // Prefer blocks of half the register file or less, so that two share an SM.
+  static constexpr int MAX_COLS = cap(WANT, LIMIT / 2) >= WANT / 2 ? cap(WANT, LIMIT / 2) : cap(WANT, LIMIT);
+  static constexpr int MAX_THREADS = MAX_COLS * M * COMPS < 32 ? 32 : MAX_COLS * M * COMPS;
+  static constexpr int MIN_BLOCKS = 65536 / (REGS * (MAX_THREADS < 128 ? 128 : MAX_THREADS));
+};
+
+template <typename T, int N, int V, int COMPS>
+int col_shape_cols(int nx, int members, int sm_count) {
+  using S = ColShape<T, N, V, COMPS>;
+  int cols = std::min(S::MAX_COLS, nx);
+  const int least = sizeof(T) == 4 ? 2 : 1;
+  while (cols > least && cols / 2 * S::M * COMPS >= 32 &&
+         static_cast<long long>(nx / cols) * members < 2LL * sm_count)
+    cols /= 2;
+  return cols;
+}
+
+inline int log2_of(int n) {
+  int l = 0;
+  while ((1 << l) < n) ++l;
+  return l;
+}
+
+}  // namespace
+}  // namespace pg

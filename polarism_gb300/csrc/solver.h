@@ -69,6 +69,8 @@ struct pg_solver {
   void* tw_y = nullptr;
   void* prop = nullptr;       // [table][member][nx + ny] propagator factors
   void* tw4 = nullptr;        // FP32 1024-point four-step factors W_1024^{n2 k1} (split_fast.cu)
+  void* reg_x = nullptr;      // W_n^{t k} tables of the register-resident passes (split_reg.cuh),
+  void* reg_y = nullptr;      // rows and columns; null where the size has no such pass
   void* split_consts = nullptr;
   std::map<std::tuple<int, int, int>, cudaGraphExec_t> split_graphs;  // (ordering, len, parity)
   void* ifrk = nullptr;       // IFRK stage buffers (created on first use)

@@ -56,20 +56,13 @@ __global__ void __launch_bounds__(1024) row_pass_kernel(typename C2T<T>::type* _
   __syncthreads();
   if (a.forward) smem_fft<T, false, false, COMP>(buf, tws, a.log2nx, a.log2rows, 1, a.nx);
   if (a.multiply) {
-    // psi (1 + dx[j]) (1 + dy[i]) scale = (psi + psi (dx + dy + dx dy)) scale, with the factor
-    // differences d stored in place of the factors (see setup_tables) and scale a power of two.
     const C2* pxm = px + static_cast<long long>(member) * a.table_stride;
     const C2* pym = py + static_cast<long long>(member) * a.table_stride;
     const T scale = static_cast<T>(a.scale);
     for (int e = threadIdx.x; e < count; e += blockDim.x) {
       const int r = e >> a.log2nx;
       const int j = e & (a.nx - 1);
-      const C2 dx = pxm[j], dy = pym[row0 + r];
-      const C2 dxy = cmul(dx, dy);
-      const C2 f1{dx.x + dy.x + dxy.x, dx.y + dy.y + dxy.y};
-      const C2 v = buf[e];
-      const C2 vf = cmul(v, f1);
-      buf[e] = C2{(v.x + vf.x) * scale, (v.y + vf.y) * scale};
+      buf[e] = kick(buf[e], pxm[j], pym[row0 + r], scale);
     }
     __syncthreads();
   }

@@ -1,4 +1,4 @@
-// Split-step passes for FP32 rows and columns of 1024 sites: register-resident four-step FFTs.
+// IFRK passes for FP32 rows and columns of 1024 sites: register-resident four-step FFTs.
 //
 // A 1024-point transform is 1024 = 32 x 32 (n = n2 + 32 n1, k = k1 + 32 k2):
 //   X[k1 + 32 k2] = sum_n2 W_32^{n2 k2} W_1024^{n2 k1} sum_n1 x[n2 + 32 n1] W_32^{n1 k1}.
@@ -132,57 +132,6 @@ __device__ __forceinline__ void fft1024_warp(float2 (&v)[32], int lane, float2* 
   dft32<false>(v);
 }
 
-// ------------------------------------------------------------------ row pass
-__global__ void __launch_bounds__(kRowWarps * 32, 2)
-    row_fast_kernel(float2* __restrict__ data, const float4* __restrict__ tw4_g,
-                    const float2* __restrict__ px, const float2* __restrict__ py,
-                    const RowPassArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (a.halt != nullptr && __ldcg(a.halt) != 0) return;  // steady-state monitor halted the run
-  float4* tw4 = reinterpret_cast<float4*>(smem_raw);                     // [32][32]
-  float2* xb = reinterpret_cast<float2*>(tw4 + kN);                      // [warps][32][33]
-  for (int i = threadIdx.x; i < kN; i += blockDim.x) tw4[i] = tw4_g[i];
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int member = blockIdx.z;
-  float2* buf = xb + warp * 32 * kXStride;
-  const float2* pxm = px + static_cast<long long>(member) * a.table_stride;
-  const float2* pym = py + static_cast<long long>(member) * a.table_stride;
-  const float scale = static_cast<float>(a.scale);
-  const long long plane = static_cast<long long>(kN) * a.ny;
-#pragma unroll 1
-  for (int q = 0; q < kRowsPerWarp; ++q) {
-    const int row = (blockIdx.x * kRowWarps + warp) * kRowsPerWarp + q;
-    float2* d = data + member * plane + static_cast<long long>(row) * kN;
-    float2 v[32];
-#pragma unroll
-    for (int t = 0; t < 32; ++t) v[t] = d[lane + 32 * t];
-    // Phase 0: forward transform and kick; phase 1: the inverse transform (conj32).
-#pragma unroll 1
-    for (int ph = 0; ph < 2; ++ph) {
-      if (ph == 0 ? a.forward : a.inverse) {
-        if (ph == 1) conj32(v);
-        fft1024_warp(v, lane, buf, tw4);
-        if (ph == 1) conj32(v);
-      }
-      if (ph == 0 && a.multiply) {
-        // psi (1 + dx) (1 + dy) scale, the factor differences stored (see split.cu)
-        const float2 dy = pym[row];
-#pragma unroll
-        for (int r = 0; r < 32; ++r) {
-          const float2 dx = pxm[lane + 32 * r];
-          const float2 dxy = cmul(dx, dy);
-          const float2 f1 = make_float2(dx.x + dy.x + dxy.x, dx.y + dy.y + dxy.y);
-          const float2 vf = cmul(v[r], f1);
-          v[r] = make_float2((v[r].x + vf.x) * scale, (v[r].y + vf.y) * scale);
-        }
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < 32; ++t) d[lane + 32 * t] = v[t];
-  }
-}
-
 // ------------------------------------------------------------------ IFRK row pass
 // ifrk_row_kernel (ifrk.cu) for FP32 rows of 1024 sites of a one-component field: the row's
 // forward transform, the stage spectrum saved, the Lawson combination
@@ -274,118 +223,6 @@ __device__ __forceinline__ void fft1024_panel(float2 (&v)[32], int p, int c, flo
   dft32<false>(v);
 }
 
-// The local step of the single case (LocalStep::single) over a panel in site order
-// ([row][column] in pan), kSiteBatch sites a thread at a time: the reservoir and envelope
-// loads of the whole batch are issued before the first site's arithmetic.  One site at a time,
-// a site's reservoir store would come before the next site's loads, which the compiler may not
-// move above it (the same array), so a thread would keep one site's loads in flight.
-constexpr int kSiteBatch = 4;  // 8 measured slightly slower
-template <int OP, bool NOISE>
-__device__ __forceinline__ void panel_local_single(const LocalStep<float>& local, float2* pan,
-                                                   int nx, int x0) {
-  const int threads = static_cast<int>(blockDim.x);
-  for (int e0 = threadIdx.x; e0 < kPanel * kN; e0 += kSiteBatch * threads) {
-    int o[kSiteBatch];
-    bool ok[kSiteBatch];
-    float2 x[kSiteBatch];
-    float n[kSiteBatch], P[kSiteBatch];
-#pragma unroll
-    for (int u = 0; u < kSiteBatch; ++u) {
-      const int e = e0 + u * threads;
-      ok[u] = e < kPanel * kN;
-      const int ee = ok[u] ? e : e0;  // a site of the panel: loads stay in bounds
-      o[u] = (ee / kPanel) * nx + x0 + ee % kPanel;
-      x[u] = pan[ee];
-      n[u] = local.rm[o[u]];
-      P[u] = local.pm[o[u]];
-    }
-#pragma unroll
-    for (int u = 0; u < kSiteBatch; ++u)
-      n[u] = local.template step_single<OP, NOISE>(x[u], n[u], P[u], o[u]);
-#pragma unroll
-    for (int u = 0; u < kSiteBatch; ++u) {
-      if (!ok[u]) continue;
-      pan[e0 + u * threads] = x[u];
-      if (OP != SPLIT_OP_NONLINEAR) local.rm[o[u]] = n[u];
-    }
-  }
-}
-
-__global__ void __launch_bounds__(kPanel * 32, 2)
-    col_fast_kernel(float2* __restrict__ data, float* __restrict__ res, const float* __restrict__ pump,
-                    const float* __restrict__ potential, const float4* __restrict__ tw4_g,
-                    const SplitConst<float>* __restrict__ consts, const float* __restrict__ scales,
-                    const unsigned long long* __restrict__ step_base, const ColPassArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (a.halt != nullptr && __ldcg(a.halt) != 0) return;  // steady-state monitor halted the run
-  float4* tw4 = reinterpret_cast<float4*>(smem_raw);  // [32][32]
-  float2* pan = reinterpret_cast<float2*>(tw4 + kN);  // exchange, or [row][c] for the local step
-  for (int i = threadIdx.x; i < kN; i += blockDim.x) tw4[i] = tw4_g[i];
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c = lane & (kPanel - 1);
-  const int p = warp * 4 + (lane >> 3);  // n2: 0..31
-  const int member = blockIdx.z;
-  const int x0 = blockIdx.x * kPanel;
-  const long long plane = static_cast<long long>(a.nx) * kN;
-  float2* d = data + member * plane + x0 + c;
-  float2 v[32];
-#pragma unroll
-  for (int t = 0; t < 32; ++t) v[t] = d[static_cast<long long>(p + 32 * t) * a.nx];
-  // Phase 0: the inverse transform (conj32 around the forward one) and the local step;
-  // phase 1: the forward transform.
-#pragma unroll 1
-  for (int ph = 0; ph < 2; ++ph) {
-    if (ph == 0 ? a.inverse : a.forward) {
-      if (ph == 0) conj32(v);
-      fft1024_panel(v, p, c, pan, tw4);
-      if (ph == 0) conj32(v);
-    }
-    if (ph == 1 || a.op == SPLIT_OP_NONE) continue;
-    // Through shared memory in site order, so that the local step is one loop.
-    __syncthreads();
-#pragma unroll
-    for (int t = 0; t < 32; ++t) pan[(p + 32 * t) * kPanel + c] = v[t];
-    __syncthreads();
-    const LocalStep<float> local(a, member, res, pump, potential, consts, scales, step_base);
-    if (local.single()) {
-      const int nx = a.nx;
-      switch (a.op * 2 + (a.noise ? 1 : 0)) {
-#define PG_SPLIT_SINGLE(OP, NOISE)             \
-  case OP * 2 + NOISE:                         \
-    panel_local_single<OP, NOISE>(local, pan, nx, x0); \
-    break;
-        PG_SPLIT_SINGLE(SPLIT_OP_KOUTER, 1)
-        PG_SPLIT_SINGLE(SPLIT_OP_KOUTER, 0)
-        PG_SPLIT_SINGLE(SPLIT_OP_NONLINEAR, 1)
-        PG_SPLIT_SINGLE(SPLIT_OP_NONLINEAR, 0)
-        PG_SPLIT_SINGLE(SPLIT_OP_RES_START, 1)
-        PG_SPLIT_SINGLE(SPLIT_OP_RES_START, 0)
-        PG_SPLIT_SINGLE(SPLIT_OP_RES_END, 1)
-        PG_SPLIT_SINGLE(SPLIT_OP_RES_END, 0)
-        PG_SPLIT_SINGLE(SPLIT_OP_RES_END_START, 1)
-        PG_SPLIT_SINGLE(SPLIT_OP_RES_END_START, 0)
-#undef PG_SPLIT_SINGLE
-        default:
-          break;
-      }
-    } else {
-#pragma unroll 2
-      for (int e = threadIdx.x; e < kPanel * kN; e += blockDim.x) {
-        const int row = e / kPanel, col = e % kPanel;
-        float2 x = pan[e];
-        local.apply(x, static_cast<long long>(row) * a.nx + x0 + col);
-        pan[e] = x;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int t = 0; t < 32; ++t) v[t] = pan[(p + 32 * t) * kPanel + c];
-  }
-#pragma unroll
-  for (int t = 0; t < 32; ++t) d[static_cast<long long>(p + 32 * t) * a.nx] = v[t];
-}
-
 // ------------------------------------------------------------------ IFRK column pass
 // ifrk_col_kernel (ifrk.cu) for FP32 columns of 1024 sites of a one-component field: the
 // forward-only pass that forms W (mode 3, any reservoir), and the stage and step-end passes
@@ -458,8 +295,6 @@ __global__ void __launch_bounds__(kPanel * 32, 2)
   for (int t = 0; t < 32; ++t) d[static_cast<long long>(p + 32 * t) * a.nx] = v[t];
 }
 
-size_t row_fast_smem() { return kN * sizeof(float4) + kRowWarps * 32 * kXStride * sizeof(float2); }
-size_t col_fast_smem() { return kN * sizeof(float4) + kPanel * kPanelStride * sizeof(float2); }
 size_t ifrk_col_fast_smem() { return kPanel * kPanelStride * sizeof(float2); }
 size_t ifrk_row_fast_smem() { return kRowWarps * 32 * kXStride * sizeof(float2); }
 
@@ -484,26 +319,11 @@ void split_fast_twiddles(float* out) {
 }
 
 cudaError_t configure_split_fast() {
-  cudaError_t e = cudaFuncSetAttribute(row_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(row_fast_smem()));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(ifrk_row_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(ifrk_row_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(ifrk_row_fast_smem()));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(ifrk_col_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(ifrk_col_fast_smem()));
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(col_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              static_cast<int>(col_fast_smem()));
-}
-
-cudaError_t launch_row_fast(float* data, const float* tw4, const float* px, const float* py,
-                            const RowPassArgs& a, int members, cudaStream_t stream) {
-  const dim3 grid(a.ny / (kRowWarps * kRowsPerWarp), 1, members);
-  row_fast_kernel<<<grid, kRowWarps * 32, row_fast_smem(), stream>>>(
-      reinterpret_cast<float2*>(data), reinterpret_cast<const float4*>(tw4),
-      reinterpret_cast<const float2*>(px), reinterpret_cast<const float2*>(py), a);
-  return cudaGetLastError();
+  return cudaFuncSetAttribute(ifrk_col_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              static_cast<int>(ifrk_col_fast_smem()));
 }
 
 bool ifrk_fast_row(const IfrkRowArgs& a) {
@@ -538,17 +358,6 @@ cudaError_t launch_ifrk_col_fast(float* psi, const float* n0, float* dn_out, flo
       reinterpret_cast<float2*>(const_cast<float*>(psi_start)),
       reinterpret_cast<float2*>(const_cast<float*>(psi_new)), pump, potential,
       reinterpret_cast<const float4*>(tw4), consts, scales, step_base, a);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_col_fast(float* data, float* res, const float* pump, const float* potential,
-                            const float* tw4, const SplitConst<float>* consts, const float* scales,
-                            const unsigned long long* step_base, const ColPassArgs& a,
-                            cudaStream_t stream) {
-  const dim3 grid(a.nx / kPanel, 1, a.members);
-  col_fast_kernel<<<grid, kPanel * 32, col_fast_smem(), stream>>>(
-      reinterpret_cast<float2*>(data), res, pump, potential, reinterpret_cast<const float4*>(tw4),
-      consts, scales, step_base, a);
   return cudaGetLastError();
 }
 

@@ -79,19 +79,31 @@ cudaError_t launch_col_pass(T* data, T* res, const T* pump, const T* potential, 
 template <typename T>
 cudaError_t configure_split_kernels(size_t max_smem);
 
-// Register-resident four-step passes for FP32 rows / columns of 1024 sites (split_fast.cu):
-// whether they apply, their W_1024^{n2 k1} table (1024 float4: rounded value, remainder),
-// attribute set-up and launches (arguments as launch_row_pass / launch_col_pass).
+// The FP32 passes on register-resident transforms (split_reg.cuh): axes of 64 to 4096 points.
+inline bool reg_fft_size(int n) { return n >= 64 && n <= 4096 && (n & (n - 1)) == 0; }
+// Values a thread holds of a transform of n points.  By size alone, so that a member's result does
+// not depend on how many are stepped with it.  Eight to 512 points: a K-outer step of one 256^2 /
+// 512^2 member 11.6 / 16.2 us against 17.9 / 21.5 with sixteen, eight 512^2 members 49.6 against
+// 50.7 (sixteen is ahead only on large batches of small grids: 25.8 against 28.0 us for sixteen
+// 256^2 members).  Above, two passes of eight do not reach n with a last DFT of at most 8.
+inline int reg_fft_vals(int n) { return n <= 512 ? 8 : 16; }
+// Attribute set-up for a grid's axes that have such passes, and launches.  tab: W_n^{t k} at entry
+// k (n / vals) + t, k < vals, as {re, im} rounded and remainders.
+cudaError_t configure_split_reg(int nx, int ny);
+cudaError_t launch_row_reg(float* data, const float* tab, const float* px, const float* py,
+                           const RowPassArgs& a, int members, int sm_count,
+                           cudaStream_t stream);
+cudaError_t launch_col_reg(float* data, float* res, const float* pump, const float* potential,
+                           const float* tab, const SplitConst<float>* consts, const float* scales,
+                           const unsigned long long* step_base, const ColPassArgs& a, int sm_count, cudaStream_t stream);
+
+// Register-resident four-step IFRK passes for FP32 rows / columns of 1024 sites (split_fast.cu):
+// whether they apply, their W_1024^{n2 k1} table (1024 float4: rounded value, remainder) and
+// attribute set-up.
 bool split_fast_row(int nx, int ny);
 bool split_fast_col(int nx, int ny);
 void split_fast_twiddles(float* out);
 cudaError_t configure_split_fast();
-cudaError_t launch_row_fast(float* data, const float* tw4, const float* px, const float* py,
-                            const RowPassArgs& a, int members, cudaStream_t stream);
-cudaError_t launch_col_fast(float* data, float* res, const float* pump, const float* potential,
-                            const float* tw4, const SplitConst<float>* consts, const float* scales,
-                            const unsigned long long* step_base, const ColPassArgs& a,
-                            cudaStream_t stream);
 
 // The IFRK row pass on the same transforms (FP32, one component, rows of 1024 sites): whether
 // it applies and its launch (arguments as launch_ifrk_row; tw4 as above).

@@ -14,6 +14,22 @@ namespace {
 __device__ __forceinline__ float mul_rn_t(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn_t(double a, double b) { return __dmul_rn(a, b); }
 
+// psi (1 + dx) (1 + dy) scale, with the factor differences d stored in place of the factors (see
+// setup_tables) and scale a power of two.  FP32 forms the combined difference first, so that
+// psi is rounded once; FP64, bound by its arithmetic, takes two products psi + psi d (10 instead of
+// 16 instructions).
+__device__ __forceinline__ float2 kick(float2 v, float2 dx, float2 dy, float scale) {
+  const float2 dxy = cmul(dx, dy);
+  const float2 f1 = make_float2(dx.x + dy.x + dxy.x, dx.y + dy.y + dxy.y);
+  const float2 vf = cmul(v, f1);
+  return make_float2((v.x + vf.x) * scale, (v.y + vf.y) * scale);
+}
+__device__ __forceinline__ double2 kick(double2 v, double2 dx, double2 dy, double scale) {
+  const double2 a = make_double2(v.x + (v.x * dx.x - v.y * dx.y), v.y + (v.x * dx.y + v.y * dx.x));
+  return make_double2((a.x + (a.x * dy.x - a.y * dy.y)) * scale,
+                      (a.y + (a.x * dy.y + a.y * dy.x)) * scale);
+}
+
 // Midpoint RK2 reservoir half step at frozen |psi|^2 with the final clamp
 // (polarism/reservoir/single_reservoir.py:100-111).
 template <typename T>
@@ -55,36 +71,62 @@ __device__ __forceinline__ void reservoir_half2(T& a, T& b, T rho, T pump, T h, 
   b = nb > T(0) ? nb : T(0);
 }
 
-// (exp(x) - 1) / x, exp(x) - 1 and (sin, cos - 1) of the local step.  FP64 follows the
-// reference (expm1 with its three-term series below 1e-6, library sincos).  FP32 uses
-// five-term series for |x| < 2^-5 (truncation x^5/720 < 5e-11 relative) and Taylor
-// polynomials for |phi| < 1/8 (truncation below 1e-13), the library functions outside: the
-// per-step arguments are that small at the time steps the split-step solvers run with, and
-// the polynomials are cheaper than the library's range reduction.
-__device__ __forceinline__ double phase_time_factor(double x) {
-  return fabs(x) < 1e-6 ? 1.0 + x * 0.5 + x * x / 6.0 : expm1(x) / x;
+// (exp(x) - 1) / x with exp(x) - 1 beside it, and (sin, cos - 1), of the local step: Taylor
+// polynomials for |x| < 2^-5 (truncated below 5e-11 relative in FP32, 8e-21 in FP64) and
+// |phi| < 1/8 (below 1e-13, 3e-21), the library functions outside.  The per-step arguments are
+// that small at the time steps the split-step solvers run with, and the polynomials are cheaper
+// than the library's range reduction and division: in FP64, whose two lanes a clock bound the
+// pass, about 25 instructions a site instead of some 90.
+__device__ __forceinline__ double expm1_over(double x, double* e) {
+  if (fabs(x) < 0.03125) {
+    double p = fma(x, 1.0 / 362880.0, 1.0 / 40320.0);
+    p = fma(x, p, 1.0 / 5040.0);
+    p = fma(x, p, 1.0 / 720.0);
+    p = fma(x, p, 1.0 / 120.0);
+    p = fma(x, p, 1.0 / 24.0);
+    p = fma(x, p, 1.0 / 6.0);
+    p = fma(x, p, 0.5);
+    p = fma(x, p, 1.0);
+    *e = x * p;
+    return p;
+  }
+  *e = expm1(x);
+  return *e / x;
 }
-__device__ __forceinline__ float phase_time_factor(float x) {
-  if (fabsf(x) < 0.03125f)
-    return 1.0f + x * (0.5f + x * (1.0f / 6.0f + x * (1.0f / 24.0f + x * (1.0f / 120.0f))));
-  return expm1f(x) / x;
-}
-__device__ __forceinline__ double local_expm1(double x) { return expm1(x); }
-__device__ __forceinline__ float local_expm1(float x) {
-  if (fabsf(x) < 0.03125f)
-    return x * (1.0f + x * (0.5f + x * (1.0f / 6.0f + x * (1.0f / 24.0f + x * (1.0f / 120.0f)))));
-  return expm1f(x);
+__device__ __forceinline__ float expm1_over(float x, float* e) {
+  if (fabsf(x) < 0.03125f) {
+    const float p = 1.0f + x * (0.5f + x * (1.0f / 6.0f + x * (1.0f / 24.0f + x * (1.0f / 120.0f))));
+    *e = x * p;
+    return p;
+  }
+  *e = expm1f(x);
+  return *e / x;
 }
 __device__ __forceinline__ void local_sincos_m1(double x, double* s, double* cm1) {
-  double c;
-  sincos(x, s, &c);
-  *cm1 = c - 1.0;
+  if (fabs(x) < 0.125) {
+    const double x2 = x * x;
+    double p = fma(x2, -1.0 / 39916800.0, 1.0 / 362880.0);
+    p = fma(x2, p, -1.0 / 5040.0);
+    p = fma(x2, p, 1.0 / 120.0);
+    p = fma(x2, p, -1.0 / 6.0);
+    *s = fma(x * x2, p, x);
+    double q = fma(x2, 1.0 / 479001600.0, -1.0 / 3628800.0);
+    q = fma(x2, q, 1.0 / 40320.0);
+    q = fma(x2, q, -1.0 / 720.0);
+    q = fma(x2, q, 1.0 / 24.0);
+    q = fma(x2, q, -0.5);
+    *cm1 = x2 * q;
+  } else {
+    double c;
+    sincos(x, s, &c);
+    *cm1 = c - 1.0;
+  }
 }
 __device__ __forceinline__ void local_sincos_m1(float x, float* s, float* cm1) {
   if (fabsf(x) < 0.125f) {
     const float x2 = x * x;
-    *s = x * (1.0f - x2 * (1.0f / 6.0f) * (1.0f - x2 * (1.0f / 20.0f) * (1.0f - x2 * (1.0f / 42.0f))));
-    *cm1 = -x2 * 0.5f * (1.0f - x2 * (1.0f / 12.0f) * (1.0f - x2 * (1.0f / 30.0f) * (1.0f - x2 * (1.0f / 56.0f))));
+    *s = fmaf(x * x2, fmaf(x2, fmaf(x2, -1.0f / 5040.0f, 1.0f / 120.0f), -1.0f / 6.0f), x);
+    *cm1 = x2 * fmaf(x2, fmaf(x2, fmaf(x2, 1.0f / 40320.0f, -1.0f / 720.0f), 1.0f / 24.0f), -0.5f);
   } else {
     float c;
     sincosf(x, s, &c);
@@ -102,12 +144,13 @@ __device__ __forceinline__ void nonlinear(T& re, T& im, T n, T n2, bool two, T v
                                           const SplitConst<T>& k) {
   const T rho = re * re + im * im;
   const T gain = (k.R * n - k.gamma_C) * T(0.5) + vim * k.inv_hbar;
-  const T x = T(2) * gain * dt;
-  const T phase_time = dt * phase_time_factor(x);
+  // (exp(2 y) - 1) / (2 y) = p (1 + e / 2) with y = gain dt, e = exp(y) - 1, p = e / y
+  T e;
+  const T p = expm1_over(gain * dt, &e);
+  const T phase_time = dt * (p + p * (T(0.5) * e));
   T pot = vre + k.g_R * n;
   if (two) pot += k.g_I * n2;
   const T phase = (pot * dt + k.g_C * rho * phase_time) * k.inv_hbar;
-  const T e = local_expm1(gain * dt);
   T s, c1;
   local_sincos_m1(phase, &s, &c1);
   const T dre = e + c1 + e * c1;
@@ -215,58 +258,73 @@ struct LocalStep {
     return n;
   }
 
-  __device__ __forceinline__ void apply(C2& v, long long o) const {
-    T n = (reservoir || two) ? rm[o] : T(0);
-    T n2 = two ? rm2[o] : T(0);
-    T Pa, Pb;  // pump at the first and the second coefficient sample
+  // What the step reads at a site of any launch: the reservoir fields, the pump at the first and
+  // the second coefficient sample, the potential.
+  struct Inputs {
+    T n, n2, Pa, Pb, vre, vim;
+  };
+  __device__ __forceinline__ Inputs load(long long o) const {
+    Inputs s;
+    s.n = (reservoir || two) ? rm[o] : T(0);
+    s.n2 = two ? rm2[o] : T(0);
     if (L > 1) {
-      Pa = pump_terms_value(pm, pump_term_stride, c0, m_count, L, o);
-      Pb = pump_terms_value(pm, pump_term_stride, c1, m_count, L, o);
+      s.Pa = pump_terms_value(pm, pump_term_stride, c0, m_count, L, o);
+      s.Pb = pump_terms_value(pm, pump_term_stride, c1, m_count, L, o);
     } else {
       const T P = pm[o];
-      Pa = mul_rn_t(s0, P);
-      Pb = mul_rn_t(s1, P);
+      s.Pa = mul_rn_t(s0, P);
+      s.Pb = mul_rn_t(s1, P);
     }
-    T vre = T(0), vim = T(0);
+    s.vre = s.vim = T(0);
     if (vm) {
-      vre = pot_kind == 2 ? vm[2 * o] : vm[o];
-      vim = pot_kind == 2 ? vm[2 * o + 1] : T(0);
+      s.vre = pot_kind == 2 ? vm[2 * o] : vm[o];
+      s.vim = pot_kind == 2 ? vm[2 * o + 1] : T(0);
     }
-    bool add_noise = false;
-    switch (op) {
-      case SPLIT_OP_KOUTER:
-        res_half(n, n2, v.x * v.x + v.y * v.y, Pa);
-        nonlinear(v.x, v.y, n, n2, two, vre, vim, dt, k);
-        res_half(n, n2, v.x * v.x + v.y * v.y, Pb);
-        add_noise = noise != 0;
-        break;
-      case SPLIT_OP_RES_START:
-        res_half(n, n2, v.x * v.x + v.y * v.y, Pa);
-        break;
-      case SPLIT_OP_RES_END_START: {
-        const T rho = v.x * v.x + v.y * v.y;
-        res_half(n, n2, rho, Pa);
-        res_half(n, n2, rho, Pb);
-        break;
-      }
-      case SPLIT_OP_NONLINEAR:
-        nonlinear(v.x, v.y, n, n2, two, vre, vim, dt, k);
-        add_noise = noise != 0;
-        break;
-      case SPLIT_OP_RES_END:
-        res_half(n, n2, v.x * v.x + v.y * v.y, Pa);
-        break;
-      default:
-        break;
+    return s;
+  }
+  // The step on those values: v and the reservoir fields of s advance.
+  template <int OP, bool NOISE>
+  __device__ __forceinline__ void compute(C2& v, Inputs& s, long long o) const {
+    const T rho = v.x * v.x + v.y * v.y;
+    if (OP == SPLIT_OP_KOUTER) {
+      res_half(s.n, s.n2, rho, s.Pa);
+      nonlinear(v.x, v.y, s.n, s.n2, two, s.vre, s.vim, dt, k);
+      res_half(s.n, s.n2, v.x * v.x + v.y * v.y, s.Pb);
+    } else if (OP == SPLIT_OP_RES_START || OP == SPLIT_OP_RES_END) {
+      res_half(s.n, s.n2, rho, s.Pa);
+    } else if (OP == SPLIT_OP_RES_END_START) {
+      res_half(s.n, s.n2, rho, s.Pa);
+      res_half(s.n, s.n2, rho, s.Pb);
+    } else if (OP == SPLIT_OP_NONLINEAR) {
+      nonlinear(v.x, v.y, s.n, s.n2, two, s.vre, s.vim, dt, k);
     }
-    if (add_noise) {
+    if (NOISE && (OP == SPLIT_OP_KOUTER || OP == SPLIT_OP_NONLINEAR)) {
       const uint32_t cell[1] = {static_cast<uint32_t>(o)};
       Words4 w[1];
       philox_cells(cell, prefix, w);
-      WignerDraw<T>::apply(w[0], k.noise_a + k.noise_b * n, v.x, v.y);
+      WignerDraw<T>::apply(w[0], k.noise_a + k.noise_b * s.n, v.x, v.y);
     }
-    if (reservoir || two) rm[o] = n;
-    if (two) rm2[o] = n2;
+  }
+  __device__ __forceinline__ void store(const Inputs& s, long long o) const {
+    if (reservoir || two) rm[o] = s.n;
+    if (two) rm2[o] = s.n2;
+  }
+  __device__ __forceinline__ void apply(C2& v, long long o) const {
+    Inputs s = load(o);
+    switch (op * 2 + (noise ? 1 : 0)) {
+#define PG_SPLIT_OP(OP)                      \
+  case OP * 2: compute<OP, false>(v, s, o); break; \
+  case OP * 2 + 1: compute<OP, true>(v, s, o); break;
+      PG_SPLIT_OP(SPLIT_OP_KOUTER)
+      PG_SPLIT_OP(SPLIT_OP_NONLINEAR)
+      PG_SPLIT_OP(SPLIT_OP_RES_START)
+      PG_SPLIT_OP(SPLIT_OP_RES_END)
+      PG_SPLIT_OP(SPLIT_OP_RES_END_START)
+#undef PG_SPLIT_OP
+      default:
+        break;
+    }
+    store(s, o);
   }
 };
 
