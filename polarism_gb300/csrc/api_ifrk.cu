@@ -65,11 +65,6 @@ int ilog2i(int n) {
   while ((1 << l) < n) ++l;
   return l;
 }
-double wavenumber(int j, int n, double d) {
-  const int k = j < (n + 1) / 2 ? j : j - n;
-  return 2.0 * kPi2 * static_cast<double>(k) / (static_cast<double>(n) * d);
-}
-
 struct IfrkBuffers {
   size_t csize = 0;
   void* W = nullptr;
@@ -82,6 +77,8 @@ struct IfrkBuffers {
   void* dn[kIfrkMaxStages] = {};
   void* tables = nullptr;
   size_t table_capacity = 0;  // number of (members x (nx + ny)) tables
+  std::vector<double> table_taus;  // what `tables` holds
+  double* rates = nullptr;    // -hbar / 2m per member
   double* partials = nullptr;
   int partial_blocks = 0;
   std::vector<double> host_partials;
@@ -122,6 +119,14 @@ int ensure_ifrk(pg_solver* s) {
   b->partial_blocks = cols_blocks;
   PG_CUDA(cudaMalloc(&b->partials, sizeof(double) * static_cast<size_t>(cols_blocks) * c.members));
   b->host_partials.resize(static_cast<size_t>(cols_blocks) * c.members);
+  if (s->comps == 1) {
+    std::vector<double> rates(c.members);
+    for (int m = 0; m < c.members; ++m) rates[m] = -s->physics[m].hbar / (2.0 * s->physics[m].m_eff);
+    PG_CUDA(cudaMalloc(&b->rates, rates.size() * sizeof(double)));
+    PG_CUDA(cudaMemcpyAsync(b->rates, rates.data(), rates.size() * sizeof(double), cudaMemcpyHostToDevice,
+                            s->stream));
+    PG_CUDA(pg::stream_sync(s));
+  }
   if (s->comps == 2) {
     std::vector<SpinorConst> host(c.members);
     for (int m = 0; m < c.members; ++m) {
@@ -146,47 +151,41 @@ int ensure_ifrk(pg_solver* s) {
     PG_CUDA(configure_ifrk_kernels<double>(200 * 1024));
   else
     PG_CUDA(configure_ifrk_kernels<float>(200 * 1024));
+  if (s->reg_x != nullptr || s->reg_y != nullptr) PG_CUDA(configure_ifrk_reg(c.nx, c.ny, s->comps));
+  if (c.precision == PG_SINGLE && s->comps == 1 && ifrk_col_fast_size(c.nx, c.ny)) {
+    std::vector<float> tw4(4 * 1024);
+    ifrk_col_fast_twiddles(tw4.data());
+    PG_CUDA(cudaMalloc(&s->tw4, tw4.size() * sizeof(float)));
+    PG_CUDA(cudaMemcpyAsync(s->tw4, tw4.data(), tw4.size() * sizeof(float), cudaMemcpyHostToDevice, s->stream));
+    PG_CUDA(configure_ifrk_col_fast());
+    PG_CUDA(pg::stream_sync(s));  // the host table goes out of scope
+  }
   (void)esize;
   return PG_OK;
 }
 
-// Upload the separable Lawson factors E(tau)/N for a list of tau values.
+// The separable Lawson factors E(tau) / N for a list of tau values, formed on the device; kept while
+// the list stays the same (a fixed step repeats it in every call).
 template <typename T>
-int upload_tables(pg_solver* s, const std::vector<double>& taus) {
+int make_tables(pg_solver* s, const std::vector<double>& taus) {
   IfrkBuffers& b = bufs(s);
   const pg_config& c = s->cfg;
-  const size_t per = static_cast<size_t>(c.nx + c.ny);
-  const size_t ntab = taus.size();
-  if (ntab > b.table_capacity) {
+  if (taus == b.table_taus) return PG_OK;
+  PG_CHECK(taus.size() <= kIfrkMaxTaus, PG_ERR_INVALID, "IFRK: too many distinct stage times");
+  if (taus.size() > b.table_capacity) {
+    b.table_taus.clear();
     cudaFree(b.tables);
     b.tables = nullptr;
-    PG_CUDA(cudaMalloc(&b.tables, ntab * c.members * per * 2 * sizeof(T)));
-    b.table_capacity = ntab;
+    b.table_capacity = 0;
+    PG_CUDA(cudaMalloc(&b.tables, taus.size() * c.members * static_cast<size_t>(c.nx + c.ny) * 2 * sizeof(T)));
+    b.table_capacity = taus.size();
   }
-  std::vector<T> host(ntab * c.members * per * 2);
-  const double N = static_cast<double>(c.nx) * c.ny;
-  for (size_t t = 0; t < ntab; ++t) {
-    for (int m = 0; m < c.members; ++m) {
-      const pg_physics& p = s->physics[m];
-      const double rate = -p.hbar / (2.0 * p.m_eff);
-      T* base = host.data() + ((t * c.members + m) * per) * 2;
-      for (int j = 0; j < c.nx; ++j) {
-        const double k = wavenumber(j, c.nx, c.dx);
-        const std::complex<double> v = std::exp(std::complex<double>(0.0, rate * taus[t] * k * k)) / N;
-        base[2 * j] = static_cast<T>(v.real());
-        base[2 * j + 1] = static_cast<T>(v.imag());
-      }
-      for (int i = 0; i < c.ny; ++i) {
-        const double k = wavenumber(i, c.ny, c.dy);
-        const std::complex<double> v = std::exp(std::complex<double>(0.0, rate * taus[t] * k * k));
-        base[2 * (c.nx + i)] = static_cast<T>(v.real());
-        base[2 * (c.nx + i) + 1] = static_cast<T>(v.imag());
-      }
-    }
-  }
-  PG_CUDA(cudaMemcpyAsync(b.tables, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice,
-                          s->stream));
-  PG_CUDA(pg::stream_sync(s));
+  LawsonTaus list{};
+  list.count = static_cast<int>(taus.size());
+  for (size_t t = 0; t < taus.size(); ++t) list.tau[t] = taus[t];
+  PG_CUDA(launch_lawson_tables(static_cast<T*>(b.tables), b.rates, list, c.members, c.nx, c.ny, c.dx, c.dy,
+                               s->stream));
+  b.table_taus = taus;
   return PG_OK;
 }
 
@@ -305,26 +304,25 @@ void set_taus(IfrkRowArgs& r, const StepTables& st) {
   }
 }
 
-// A row pass: the register-resident four-step form for FP32 one-component rows of 1024 sites,
-// the generic Stockham pass otherwise.
+// A row pass: on the register-resident transforms (FP32, 64 to 4096 sites), or the generic
+// Stockham pass.
 template <typename T>
 cudaError_t ifrk_row(pg_solver* s, const T* in, T* save, T* out, const T* tables,
                      const IfrkRowArgs& a, const T* tw) {
   if constexpr (sizeof(T) == 4) {
-    if (s->tw4 != nullptr && ifrk_fast_row(a))
-      return launch_ifrk_row_fast(in, save, out, tables, static_cast<const float*>(s->tw4), a,
-                                  s->stream);
+    if (s->reg_x != nullptr)
+      return launch_ifrk_row_reg(in, save, out, tables, static_cast<const float*>(s->reg_x), a,
+                                 s->sm_count, s->stream);
   }
   return launch_ifrk_row<T>(in, save, out, tables, a, tw, s->stream);
 }
 
-// A column pass: the register-resident form for FP32 one-component columns of 1024 sites
-// (the forward-only pass, and stages and step ends with one single reservoir and one laser),
-// the generic Stockham pass otherwise.
+// A column pass likewise; columns of 1024 sites in the single configuration have a pass of their own
+// (see ifrk_col_fast.cu for the measured comparison).
 template <typename T>
 cudaError_t ifrk_col(pg_solver* s, T* psi, const T* n0, T* dn_out, T* n_out, const T* psi_start,
                      const T* psi_new, const T* tw, const SplitConst<T>* consts, const T* scales,
-                     const IfrkColArgs& a) {
+                     double* partials, const IfrkColArgs& a) {
   if constexpr (sizeof(T) == 4) {
     if (s->tw4 != nullptr && ifrk_fast_col(a))
       return launch_ifrk_col_fast(psi, n0, dn_out, n_out, psi_start, psi_new,
@@ -332,10 +330,16 @@ cudaError_t ifrk_col(pg_solver* s, T* psi, const T* n0, T* dn_out, T* n_out, con
                                   static_cast<const float*>(s->potential),
                                   static_cast<const float*>(s->tw4), consts, scales, s->step_base,
                                   a, s->stream);
+    if (s->reg_y != nullptr)
+      return launch_ifrk_col_reg(psi, n0, dn_out, n_out, psi_start, psi_new,
+                                 static_cast<const float*>(s->pump),
+                                 static_cast<const float*>(s->potential),
+                                 static_cast<const float*>(s->reg_y), consts, scales, s->step_base,
+                                 partials, a, s->sm_count, s->stream);
   }
   return launch_ifrk_col<T>(psi, n0, dn_out, n_out, psi_start, psi_new,
                             static_cast<const T*>(s->pump), static_cast<const T*>(s->potential), tw,
-                            consts, scales, s->step_base, nullptr, a, s->stream);
+                            consts, scales, s->step_base, partials, a, s->stream);
 }
 
 template <typename T>
@@ -357,7 +361,7 @@ int run_step(pg_solver* s, const Plan& p, const Tableau& tb, const StepTables& s
     a.mode = 3;
     a.inverse = 0;
     a.forward = 1;
-    PG_CUDA(ifrk_col<T>(s, W, n0, nullptr, nullptr, nullptr, nullptr, tw_y, consts, nullptr, a));
+    PG_CUDA(ifrk_col<T>(s, W, n0, nullptr, nullptr, nullptr, nullptr, tw_y, consts, nullptr, nullptr, a));
     b.w_valid = true;
     s->last_launches += 1;
   }
@@ -395,7 +399,7 @@ int run_step(pg_solver* s, const Plan& p, const Tableau& tb, const StepTables& s
     a.scale_index = scale_base + i;
     PG_CUDA(ifrk_col<T>(s, W, n0, static_cast<T*>(b.dn[i]), nullptr,
                         adaptive && i == 0 ? static_cast<T*>(b.psi_start) : nullptr, nullptr, tw_y,
-                        consts, scales, a));
+                        consts, scales, nullptr, a));
     s->last_launches += 2;
   }
   // Final combination.
@@ -431,7 +435,7 @@ int run_step(pg_solver* s, const Plan& p, const Tableau& tb, const StepTables& s
       ++a.terms;
     }
     PG_CUDA(ifrk_col<T>(s, W, n0, nullptr, static_cast<T*>(b.n_new), nullptr,
-                        static_cast<T*>(b.psi_new), tw_y, consts, scales, a));
+                        static_cast<T*>(b.psi_new), tw_y, consts, scales, nullptr, a));
     s->last_launches += 2;
   }
   if (adaptive) {
@@ -464,12 +468,13 @@ int run_step(pg_solver* s, const Plan& p, const Tableau& tb, const StepTables& s
       a.coef[a.terms] = h * w;
       ++a.terms;
     }
-    PG_CUDA(launch_ifrk_col<T>(static_cast<T*>(b.ehat), n0, nullptr, static_cast<T*>(b.n_new),
-                               static_cast<T*>(b.psi_start), static_cast<T*>(b.psi_new),
-                               static_cast<const T*>(s->pump), static_cast<const T*>(s->potential),
-                               tw_y, consts, scales, s->step_base, b.partials, a, s->stream));
+    PG_CUDA(ifrk_col<T>(s, static_cast<T*>(b.ehat), n0, nullptr, static_cast<T*>(b.n_new),
+                        static_cast<T*>(b.psi_start), static_cast<T*>(b.psi_new), tw_y, consts, scales,
+                        b.partials, a));
     s->last_launches += 2;
-    const int panels = s->cfg.nx / p.col.cols;
+    const int panels = sizeof(T) == 4 && s->reg_y != nullptr
+                           ? ifrk_reg_panels(s->cfg.nx, s->cfg.ny, s->comps, s->cfg.members, s->sm_count)
+                           : s->cfg.nx / p.col.cols;
     const size_t count = static_cast<size_t>(panels) * s->cfg.members;
     PG_CUDA(cudaMemcpyAsync(b.host_partials.data(), b.partials, count * sizeof(double),
                             cudaMemcpyDeviceToHost, s->stream));
@@ -501,7 +506,7 @@ int ifrk_advance_t(pg_solver* s, int tab, int64_t start_step, int n_steps, const
   const Plan p = make_plan(s);
   const double h = s->cfg.dt;
   StepTables st = build_tables(tb, h);
-  int rc = s->comps == 1 ? upload_tables<T>(s, st.taus) : PG_OK;
+  int rc = s->comps == 1 ? make_tables<T>(s, st.taus) : PG_OK;
   if (rc != PG_OK) return rc;
   IfrkBuffers& b = bufs(s);
   b.w_valid = false;
@@ -532,7 +537,7 @@ int ifrk_trial_t(pg_solver* s, int tab, double h, const double* scales, double r
   PG_CHECK(tb.embedded, PG_ERR_INVALID, "pg_ifrk_trial: the tableau has no embedded pair");
   const Plan p = make_plan(s);
   StepTables st = build_tables(tb, h);
-  int rc = s->comps == 1 ? upload_tables<T>(s, st.taus) : PG_OK;
+  int rc = s->comps == 1 ? make_tables<T>(s, st.taus) : PG_OK;
   if (rc != PG_OK) return rc;
   rc = stage_coefficients(s, scales, 1, tb.stages * s->pump_terms, 0);
   if (rc != PG_OK) return rc;
@@ -566,6 +571,7 @@ void ifrk_release(pg_solver* s) {
   cudaFree(b->psi_start);
   cudaFree(b->n_new);
   cudaFree(b->tables);
+  cudaFree(b->rates);
   cudaFree(b->partials);
   cudaFree(b->spin);
   cudaFree(b->spin_modes);

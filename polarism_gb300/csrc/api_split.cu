@@ -121,15 +121,6 @@ int setup_tables(pg_solver* s) {
     PG_CUDA(cudaMemcpyAsync(dst, tab.data(), tab.size() * sizeof(T), cudaMemcpyHostToDevice, s->stream));
   }
   if (s->reg_x != nullptr || s->reg_y != nullptr) PG_CUDA(configure_split_reg(nx, ny));
-  if (sizeof(T) == 4 && (split_fast_row(nx, ny) || split_fast_col(nx, ny))) {
-    std::vector<float> tw4(4 * 1024);
-    split_fast_twiddles(tw4.data());
-    PG_CUDA(cudaMalloc(&s->tw4, tw4.size() * sizeof(float)));
-    PG_CUDA(cudaMemcpyAsync(s->tw4, tw4.data(), tw4.size() * sizeof(float), cudaMemcpyHostToDevice,
-                            s->stream));
-    PG_CUDA(configure_split_fast());
-    PG_CUDA(pg::stream_sync(s));  // the host tables go out of scope
-  }
   PG_CUDA(pg::stream_sync(s));
   return PG_OK;
 }

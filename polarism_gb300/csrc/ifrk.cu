@@ -13,6 +13,7 @@
 #include "fft.cuh"
 #include "ifrk_internal.h"
 #include "ifrk_sites.cuh"
+#include "spin_factor.cuh"
 #include "philox.cuh"
 #include "pg_internal.h"
 
@@ -28,23 +29,6 @@ __device__ __forceinline__ void sincos_angle(double a, float* s, float* c) {
   sincosf(static_cast<float>(fma(-n, kTwoPi, a)), s, c);
 }
 __device__ __forceinline__ void sincos_angle(double a, double* s, double* c) { sincos(a, s, c); }
-
-// sin and cos of (r_hi + r_lo)(t_hi + t_lo): the product is formed as p + t with the exact
-// rounding error of p = r_hi t_hi (an FMA) and the cross terms, reduced by 2 pi split into two
-// floats (Cody and Waite's method), so the reduced angle carries an absolute error of a few
-// 1e-7 for any angle below 2^24 turns -- the accuracy of the FP64 reduction rounded to FP32.
-__device__ __forceinline__ void sincos_product(float r_hi, float r_lo, float t_hi, float t_lo,
-                                               float* s, float* c) {
-  constexpr float kTwoPiHi = 6.28318548202514648f;        // float(2 pi)
-  constexpr float kTwoPiLo = -1.74845553146951617e-07f;   // 2 pi - kTwoPiHi
-  constexpr float kInvTwoPi = 0.159154943091895336f;
-  const float p = r_hi * t_hi;
-  const float e = fmaf(r_hi, t_hi, -p);
-  const float t = fmaf(r_hi, t_lo, fmaf(r_lo, t_hi, e));
-  const float n = rintf(p * kInvTwoPi);
-  const float d = fmaf(-n, kTwoPiLo, fmaf(-n, kTwoPiHi, p)) + t;
-  sincosf(d, s, c);
-}
 
 // Per-mode FP32 table of the two-component Lawson factor, formed once in FP64.
 __global__ void spin_mode_table_kernel(float* __restrict__ table, const SpinorConst* __restrict__ consts,
@@ -73,6 +57,26 @@ __global__ void spin_mode_table_kernel(float* __restrict__ table, const SpinorCo
     tm[5 * plane + e] = static_cast<float>(-2.0 * sc.beta * kx * ky);
     tm[6 * plane + e] = omega > 0.0 ? static_cast<float>(1.0 / omega) : 0.0f;
   }
+}
+
+// One value of the Lawson tables a thread.  On the host the same list took half a millisecond a
+// trial at 1024^2 (22 stage times of Dormand-Prince, a copy and a wait), as long as the passes.
+template <typename T>
+__global__ void lawson_tables_kernel(typename C2T<T>::type* __restrict__ tables,
+                                     const double* __restrict__ rates, const LawsonTaus taus, int nx,
+                                     int ny, double dx, double dy) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nx + ny) return;
+  const int member = blockIdx.y, t = blockIdx.z;
+  const bool row = i < nx;
+  const int n = row ? nx : ny, j = row ? i : i - nx;
+  const double d = row ? dx : dy;
+  const double k = kTwoPi * static_cast<double>(j < (n + 1) / 2 ? j : j - n) / (static_cast<double>(n) * d);
+  double s, c;
+  sincos(rates[member] * taus.tau[t] * k * k, &s, &c);
+  const double norm = row ? static_cast<double>(nx) * ny : 1.0;
+  tables[(static_cast<long long>(t) * gridDim.y + member) * (nx + ny) + i] = {static_cast<T>(c / norm),
+                                                                              static_cast<T>(s / norm)};
 }
 
 template <typename T>
@@ -143,17 +147,10 @@ __global__ void __launch_bounds__(1024) ifrk_row_kernel(const typename C2T<T>::t
       const float* tm = a.modes + static_cast<long long>(member) * kSpinModeFields * mplane +
                         static_cast<long long>(row0) * a.nx;
       for (int e = threadIdx.x; e < count; e += blockDim.x) {
-        const float re_hi = tm[e], re_lo = tm[mplane + e];
-        const float rw_hi = tm[2 * mplane + e], rw_lo = tm[3 * mplane + e];
-        const float ure = tm[4 * mplane + e], uim = tm[5 * mplane + e];
-        const float inv_om = tm[6 * mplane + e];
+        const SpinMode mode = load_spin_mode(tm + e, mplane);
         C2 acc0{T(0), T(0)}, acc1{T(0), T(0)};
 #pragma unroll 1
         for (int t = 0; t < a.terms; ++t) {
-          T se, ce, sw, cw;
-          sincos_product(re_hi, re_lo, a.tau_hi[t], a.tau_lo[t], &se, &ce);
-          sincos_product(rw_hi, rw_lo, a.tau_hi[t], a.tau_lo[t], &sw, &cw);
-          const T so = inv_om > 0.0f ? sw * inv_om : a.tau_hi[t] * inv_hbar_f;
           C2 s0, s1;
           if (a.src[t]) {
             const C2* src = static_cast<const C2*>(a.src[t]) + moff;
@@ -163,16 +160,8 @@ __global__ void __launch_bounds__(1024) ifrk_row_kernel(const typename C2T<T>::t
             s0 = buf[e];
             s1 = buf[count + e];
           }
-          const T sz = so * zf;
-          const C2 a0{cw * s0.x + sz * s0.y + so * (uim * s1.x + ure * s1.y),
-                      cw * s0.y - sz * s0.x + so * (uim * s1.y - ure * s1.x)};
-          const C2 a1{cw * s1.x - sz * s1.y + so * (ure * s0.y - uim * s0.x),
-                      cw * s1.y + sz * s1.x - so * (ure * s0.x + uim * s0.y)};
-          const T w = static_cast<T>(a.coef[t] * a.inv_n);
-          acc0.x += w * (ce * a0.x + se * a0.y);
-          acc0.y += w * (ce * a0.y - se * a0.x);
-          acc1.x += w * (ce * a1.x + se * a1.y);
-          acc1.y += w * (ce * a1.y - se * a1.x);
+          spin_term(mode, a.tau_hi[t], a.tau_lo[t], static_cast<T>(a.coef[t] * a.inv_n), zf, inv_hbar_f,
+                    s0, s1, acc0, acc1);
         }
         buf[e] = acc0;
         buf[count + e] = acc1;
@@ -231,16 +220,6 @@ __global__ void __launch_bounds__(1024) ifrk_row_kernel(const typename C2T<T>::t
     const int c = e >= count ? 1 : 0;
     out[moff + c * plane + (e - c * count)] = buf[e];
   }
-}
-
-template <typename T>
-__device__ __forceinline__ T scaled_square(T mag, T scale) {
-  // (mag / scale)^2 with the reference's handling of a zero scale.
-  if (scale > T(0)) {
-    const T r = mag / scale;
-    return r * r;
-  }
-  return mag == T(0) ? T(0) : T(INFINITY);
 }
 
 // Column pass over a panel of `cols` columns of every component of one member.  Reservoir
@@ -313,9 +292,11 @@ __global__ void __launch_bounds__(1024) ifrk_col_kernel(typename C2T<T>::type* _
     const bool batched = ifrk_sites_batched(a) && plane <= 0x7fffffffLL;
     if (batched)
       ifrk_sites_run<T, sizeof(T) == 4 ? 3 : 2, sizeof(T) == 4 ? 2 : 1>(
-          buf, C, a.log2cols, a.ny, a, k, x0, static_cast<long long>(member) * plane, n0, dn_out,
-          n_out, psi_start, psi_new, pm, vm, s0, prefix[0]);
+          buf, PanelSites{C, a.log2cols, a.nx, x0, count}, a, k, static_cast<long long>(member) * plane,
+          n0, dn_out, n_out, psi_start, psi_new, pm, vm, s0, prefix[0]);
     // Every other configuration: a site at a time.
+    const IfrkGeneral<T> general{a,  k,  s0, cs, pm, vm, n0, dn_out, n_out, psi_start, psi_new, fbase,
+                                 plane, prefix};
     if (!batched)
     for (int e = threadIdx.x; e < count; e += blockDim.x) {
       const int c = e & (C - 1), i = e >> a.log2cols;
@@ -340,96 +321,10 @@ __global__ void __launch_bounds__(1024) ifrk_col_kernel(typename C2T<T>::type* _
         dsum[q] = acc;
         nval[q] = n0[ridx[q]] + acc;
       }
-      if (a.mode == 0) {
-        T rho[2];
-#pragma unroll
-        for (int comp = 0; comp < 2; ++comp) {
-          rho[comp] = v[comp].x * v[comp].x + v[comp].y * v[comp].y;
-          if (comp < comps && psi_start) psi_start[fbase + comp * plane + o] = v[comp];
-        }
-        T vre = T(0), vim = T(0);
-        if (vm) {
-          vre = a.potential == 2 ? vm[2 * o] : vm[o];
-          vim = a.potential == 2 ? vm[2 * o + 1] : T(0);
-        }
-#pragma unroll
-        for (int comp = 0; comp < 2; ++comp) {
-          if (comp >= comps) break;
-          const int ra = Cr == comps ? comp : 0;
-          const T nA = F >= 1 ? nval[ra] : T(0);
-          const T nI = F == 2 ? nval[Cr + ra] : T(0);
-          // rhs = (-i/hbar) (V_re + g_C rho + alpha_2 rho_other + g_R n_A + g_I n_I) psi
-          //       + (R n_A - gamma_C)/2 psi + (V_im / hbar) psi
-          T eff = vre + k.g_C * rho[comp] + k.g_R * nA;
-          if (comps == 2) eff += k.alpha_2 * rho[1 - comp];
-          if (F == 2) eff += k.g_I * nI;
-          const T e_over = eff * k.inv_hbar;
-          const T g = T(0.5) * (k.R * nA - k.gamma_C) + vim * k.inv_hbar;
-          buf[i * CC + comp * C + c] = C2{g * v[comp].x + e_over * v[comp].y, g * v[comp].y - e_over * v[comp].x};
-        }
-        if (F >= 1) {
-          const T p_site = L > 1 && cs ? pump_terms_value(pm, a.pump_term_stride, cs, a.members, L, o)
-                                       : mul_rn_i(s0, pm[o]);
-#pragma unroll
-          for (int cr = 0; cr < 2; ++cr) {
-            if (cr >= Cr) break;
-            const T rr = Cr == comps ? rho[cr] : (comps == 2 ? rho[0] + rho[1] : rho[0]);
-            const T P = Cr == 2 ? mul_rn_i(p_site, k.weight[cr]) : p_site;
-            if (F == 1) {
-              dn_out[ridx[cr]] = P - (k.gamma_R + k.R * rr) * nval[cr];
-            } else if (a.res_kind == PG_RES_QDOUBLE) {
-              // quadratic_double_reservoir.py:13-14: n_R fed by kappa n_I^2.
-              const T nR = nval[cr], nI = nval[Cr + cr];
-              const T transfer = k.kappa * nI * nI;
-              dn_out[ridx[cr]] = transfer - k.gamma_R * nR - k.R * nR * rr;
-              dn_out[ridx[Cr + cr]] = P - transfer - k.gamma_I * nI;
-            } else {
-              const T nA = nval[cr], nI = nval[Cr + cr];
-              dn_out[ridx[Cr + cr]] = P - (k.gamma_I + k.R_IA) * nI + k.R_AI * nA;
-              dn_out[ridx[cr]] = k.R_IA * nI - (k.gamma_A + k.R_AI + k.R * rr) * nA;
-            }
-          }
-        }
-      } else if (a.mode == 1) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (q >= NQ) break;
-          nval[q] = nval[q] > T(0) ? nval[q] : T(0);
-          n_out[ridx[q]] = nval[q];
-        }
-#pragma unroll
-        for (int comp = 0; comp < 2; ++comp) {
-          if (comp >= comps) break;
-          C2 w = v[comp];
-          if (a.noise) {
-            const T nA = F >= 1 ? nval[Cr == comps ? comp : 0] : T(0);
-            const uint32_t cell[1] = {static_cast<uint32_t>(o)};
-            Words4 w1[1];
-            philox_cells(cell, prefix[comp], w1);
-            const Words4 words = w1[0];
-            WignerDraw<T>::apply(words, k.noise_a + k.noise_b * nA, w.x, w.y);
-            buf[i * CC + comp * C + c] = w;
-          }
-          psi_new[fbase + comp * plane + o] = w;
-        }
-      } else {  // mode 2: error norm, v = condensate error, dsum = reservoir error
-#pragma unroll
-        for (int comp = 0; comp < 2; ++comp) {
-          if (comp >= comps) break;
-          const C2 y0 = psi_start[fbase + comp * plane + o];
-          const C2 y1 = psi_new[fbase + comp * plane + o];
-          const T a0 = sqrt(y0.x * y0.x + y0.y * y0.y), a1 = sqrt(y1.x * y1.x + y1.y * y1.y);
-          const T scale = static_cast<T>(a.atol) + static_cast<T>(a.rtol) * (a0 > a1 ? a0 : a1);
-          local += static_cast<double>(
-              scaled_square(sqrt(v[comp].x * v[comp].x + v[comp].y * v[comp].y), scale));
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (q >= NQ) break;
-          const T r0 = fabs(n0[ridx[q]]), r1 = fabs(n_out[ridx[q]]);
-          const T rs = static_cast<T>(a.atol) + static_cast<T>(a.rtol) * (r0 > r1 ? r0 : r1);
-          local += static_cast<double>(scaled_square(fabs(dsum[q]), rs));
-        }
+      general.apply(v, nval, dsum, ridx, o, local);
+      if (a.mode == 0 || (a.mode == 1 && a.noise)) {
+        buf[i * CC + c] = v[0];
+        if (comps == 2) buf[i * CC + C + c] = v[1];
       }
     }
     __syncthreads();
@@ -512,6 +407,23 @@ template cudaError_t launch_ifrk_col<double>(double*, const double*, double*, do
                                              const IfrkColArgs&, cudaStream_t);
 template cudaError_t configure_ifrk_kernels<float>(size_t);
 template cudaError_t configure_ifrk_kernels<double>(size_t);
+
+template <typename T>
+cudaError_t launch_lawson_tables_t(T* tables, const double* rates, const LawsonTaus& taus, int members,
+                                   int nx, int ny, double dx, double dy, cudaStream_t stream) {
+  const dim3 grid((nx + ny + 127) / 128, members, taus.count);
+  lawson_tables_kernel<T><<<grid, 128, 0, stream>>>(reinterpret_cast<typename C2T<T>::type*>(tables), rates,
+                                                    taus, nx, ny, dx, dy);
+  return cudaGetLastError();
+}
+cudaError_t launch_lawson_tables(float* tables, const double* rates, const LawsonTaus& taus, int members,
+                                 int nx, int ny, double dx, double dy, cudaStream_t stream) {
+  return launch_lawson_tables_t(tables, rates, taus, members, nx, ny, dx, dy, stream);
+}
+cudaError_t launch_lawson_tables(double* tables, const double* rates, const LawsonTaus& taus, int members,
+                                 int nx, int ny, double dx, double dy, cudaStream_t stream) {
+  return launch_lawson_tables_t(tables, rates, taus, members, nx, ny, dx, dy, stream);
+}
 
 cudaError_t launch_spin_mode_table(float* table, const SpinorConst* consts, int nx, int ny,
                                    int members, double kx_unit, double ky_unit, cudaStream_t stream) {

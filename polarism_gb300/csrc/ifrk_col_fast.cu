@@ -1,22 +1,23 @@
-// IFRK passes for FP32 rows and columns of 1024 sites: register-resident four-step FFTs.
+// IFRK column pass for FP32 columns of 1024 sites of a one-component field with one single
+// reservoir and one laser: register-resident four-step FFTs with 32 values a thread.
 //
 // A 1024-point transform is 1024 = 32 x 32 (n = n2 + 32 n1, k = k1 + 32 k2):
 //   X[k1 + 32 k2] = sum_n2 W_32^{n2 k2} W_1024^{n2 k1} sum_n1 x[n2 + 32 n1] W_32^{n1 k1}.
 // A thread holds the 32 values x[n2 + 32 n1] of its n2 (n1 = register index), does the inner
-// 32-point DFT in registers, multiplies by W_1024^{n2 k1}, exchanges once through shared
-// memory so that it holds the 32 values of one k1, and does the outer 32-point DFT: it ends
-// with X[k1 + 32 k2] (k2 = register index), the same layout it started from, so the kinetic
-// factor and the local step apply in place.  One exchange per transform replaces the generic
-// kernel's five barrier-separated radix-4 passes through shared memory (split.cu).
+// 32-point DFT in registers, multiplies by W_1024^{n2 k1}, exchanges once through shared memory so
+// that it holds the 32 values of one k1, and does the outer 32-point DFT: it ends with
+// X[k1 + 32 k2] (k2 = register index), the layout it started from.  A block takes a panel of
+// eight columns (thread = (column, n2)); between the inverse and forward transforms the site
+// step (ifrk_sites.cuh) runs over the panel in shared memory.
 //
-// Rows: a warp per row (lane = n2), the exchange within the warp.  Columns: a block per panel
-// of eight columns (thread = (column, n2)), the exchange across the block, and between the
-// inverse and forward transforms the local step (split_local.cuh) runs over the panel in
-// shared memory as a plain loop, so its code exists once.
+// Why this pass beside ifrk_reg.cu's: its site step has up to seven loads a site and little
+// arithmetic, so it is bound by loads in flight; 128 registers a thread hold batches of eight
+// sites unspilled, 64 hold two.  A fixed step of 8 x 1024^2 takes 913 us with this column pass and
+// 1041 with the sixteen-value one, of 1024^2 x 1 164 against 179.  (The split-step column pass,
+// bound by its arithmetic, is faster on sixteen values.)
 //
 // Precision: every twiddle that is not +-1 or +-i is applied as a rounded value plus its
-// remainder (the 32-point constants and the table W_1024^{n2 k1}), as the generic FP32 passes
-// do: rounded factors alone carry a per-step amplitude bias that drifts the norm over long runs.
+// remainder (the 32-point constants and the table W_1024^{n2 k1}).
 #include <cmath>
 
 #include "ifrk_internal.h"
@@ -27,8 +28,6 @@ namespace pg {
 namespace {
 
 constexpr int kN = 1024;
-constexpr int kRowsPerWarp = 4;             // rows a warp transforms in turn (row pass)
-constexpr int kRowWarps = 8;                // warps a block (row pass)
 constexpr int kPanel = 8;                   // columns a block (column pass)
 constexpr int kXStride = 33;                // padded row of the 32 x 32 exchange
 constexpr int kPanelStride = 32 * 33 + 4;   // one column's exchange block (elements = 4 mod 16)
@@ -118,96 +117,6 @@ __device__ __forceinline__ void four_step_first(float2 (&v)[32], int n2, const f
   }
 }
 
-// A forward 1024-point transform of a row held by a warp (lane = n2, buf: 32 x kXStride
-// values).
-__device__ __forceinline__ void fft1024_warp(float2 (&v)[32], int lane, float2* buf,
-                                             const float4* tw4) {
-  four_step_first<false>(v, lane, tw4);
-#pragma unroll
-  for (int k1 = 0; k1 < 32; ++k1) buf[k1 * kXStride + lane] = v[k1];
-  __syncwarp();
-#pragma unroll
-  for (int n2 = 0; n2 < 32; ++n2) v[n2] = buf[lane * kXStride + n2];
-  __syncwarp();
-  dft32<false>(v);
-}
-
-// ------------------------------------------------------------------ IFRK row pass
-// ifrk_row_kernel (ifrk.cu) for FP32 rows of 1024 sites of a one-component field: the row's
-// forward transform, the stage spectrum saved, the Lawson combination
-// sum_t coef_t Ex_t[kx] Ey_t[ky] src_t (src_t: this row's spectrum, or a stored one), the
-// inverse transform; a warp per row, as row_fast_kernel.
-__global__ void __launch_bounds__(kRowWarps * 32, 2)
-    ifrk_row_fast_kernel(const float2* __restrict__ in, float2* __restrict__ save,
-                         float2* __restrict__ out, const float2* __restrict__ tables,
-                         const float4* __restrict__ tw4_g, const IfrkRowArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  // The twiddle table through L1, as in the IFRK column pass (no block barrier either).
-  const float4* tw4 = tw4_g;                                             // [32][32]
-  float2* xb = reinterpret_cast<float2*>(smem_raw);                      // [warps][32][33]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int member = blockIdx.z;
-  float2* buf = xb + warp * 32 * kXStride;
-  const long long table_stride = static_cast<long long>(a.members) * (kN + a.ny);
-#pragma unroll 1
-  for (int q = 0; q < kRowsPerWarp; ++q) {
-    const int row = (blockIdx.x * kRowWarps + warp) * kRowsPerWarp + q;
-    const long long moff = member * a.member_stride + static_cast<long long>(row) * kN;
-    float2 v[32];
-#pragma unroll
-    for (int t = 0; t < 32; ++t) v[t] = in ? in[moff + lane + 32 * t] : make_float2(0.f, 0.f);
-    // Phase 0: forward transform, save, combination; phase 1: the inverse transform (conj32).
-#pragma unroll 1
-    for (int ph = 0; ph < 2; ++ph) {
-      if (ph == 0 ? a.forward : a.inverse) {
-        if (ph == 1) conj32(v);
-        fft1024_warp(v, lane, buf, tw4);
-        if (ph == 1) conj32(v);
-      }
-      if (ph == 1) continue;
-      if (save) {
-#pragma unroll
-        for (int r = 0; r < 32; ++r) save[moff + lane + 32 * r] = v[r];
-      }
-      // The term on this row's own spectrum (src null; at most one) first, in place, then the
-      // stored spectra, a term at a time so that the row stays the only array in registers.
-      int own = -1;
-      for (int s = 0; s < a.terms; ++s)
-        if (a.src[s] == nullptr) own = s;
-      const float2* tabs = tables + static_cast<long long>(member) * (kN + a.ny);
-      if (own >= 0) {
-        const float2* tab = tabs + a.table[own] * table_stride;
-        const float2 ey = tab[kN + row];
-        const float c = static_cast<float>(a.coef[own]);
-#pragma unroll
-        for (int r = 0; r < 32; ++r) {
-          const float2 ev = cmul(cmul(tab[lane + 32 * r], ey), v[r]);
-          v[r] = make_float2(c * ev.x, c * ev.y);
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < 32; ++r) v[r] = make_float2(0.f, 0.f);
-      }
-#pragma unroll 1
-      for (int s = 0; s < a.terms; ++s) {
-        if (s == own) continue;
-        const float2* tab = tabs + a.table[s] * table_stride;
-        const float2* src = static_cast<const float2*>(a.src[s]) + moff;
-        const float2 ey = tab[kN + row];
-        const float c = static_cast<float>(a.coef[s]);
-#pragma unroll
-        for (int r = 0; r < 32; ++r) {
-          const float2 ev = cmul(cmul(tab[lane + 32 * r], ey), src[lane + 32 * r]);
-          v[r].x += c * ev.x;
-          v[r].y += c * ev.y;
-        }
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < 32; ++t) out[moff + lane + 32 * t] = v[t];
-  }
-}
-
 // ------------------------------------------------------------------ column pass
 // A forward 1024-point transform of the block's eight columns (thread = (column c, n2 = p));
 // pan is the panel's exchange buffer ([c][k1][n2], columns kPanelStride apart).
@@ -282,8 +191,8 @@ __global__ void __launch_bounds__(kPanel * 32, 2)
       const PhiloxCellPrefix prefix = philox_cell_prefix(
           static_cast<uint32_t>(step), static_cast<uint32_t>(step >> 32), 1u,
           static_cast<uint32_t>(k.seed), static_cast<uint32_t>(k.seed >> 32));
-      ifrk_sites_run<float, kIfrkBatch, kIfrkEndBatch>(pan, kPanel, 3, kN, a, k, x0,
-                                                       member * plane, n0, dn_out, n_out,
+      ifrk_sites_run<float, kIfrkBatch, kIfrkEndBatch>(pan, PanelSites{kPanel, 3, a.nx, x0, kPanel * kN}, a,
+                                                       k, member * plane, n0, dn_out, n_out,
                                                        psi_start, psi_new, pm, vm, s0, prefix);
     }
     __syncthreads();
@@ -296,14 +205,12 @@ __global__ void __launch_bounds__(kPanel * 32, 2)
 }
 
 size_t ifrk_col_fast_smem() { return kPanel * kPanelStride * sizeof(float2); }
-size_t ifrk_row_fast_smem() { return kRowWarps * 32 * kXStride * sizeof(float2); }
 
 }  // namespace
 
-bool split_fast_row(int nx, int ny) { return nx == kN && ny % (kRowWarps * kRowsPerWarp) == 0; }
-bool split_fast_col(int nx, int ny) { return ny == kN && nx % kPanel == 0; }
+bool ifrk_col_fast_size(int nx, int ny) { return ny == kN && nx % kPanel == 0; }
 
-void split_fast_twiddles(float* out) {
+void ifrk_col_fast_twiddles(float* out) {
   // tw4[k1][n2] = W_1024^{n2 k1}: rounded value and remainder, from double precision.
   const double pi = 3.141592653589793238462643383279502884;
   for (int k1 = 0; k1 < 32; ++k1)
@@ -318,26 +225,9 @@ void split_fast_twiddles(float* out) {
     }
 }
 
-cudaError_t configure_split_fast() {
-  cudaError_t e = cudaFuncSetAttribute(ifrk_row_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(ifrk_row_fast_smem()));
-  if (e != cudaSuccess) return e;
+cudaError_t configure_ifrk_col_fast() {
   return cudaFuncSetAttribute(ifrk_col_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               static_cast<int>(ifrk_col_fast_smem()));
-}
-
-bool ifrk_fast_row(const IfrkRowArgs& a) {
-  return a.comps == 1 && !a.spinor && a.nx == kN && a.ny % (kRowWarps * kRowsPerWarp) == 0;
-}
-
-cudaError_t launch_ifrk_row_fast(const float* in, float* save, float* out, const float* tables,
-                                 const float* tw4, const IfrkRowArgs& a, cudaStream_t stream) {
-  const dim3 grid(a.ny / (kRowWarps * kRowsPerWarp), 1, a.members);
-  ifrk_row_fast_kernel<<<grid, kRowWarps * 32, ifrk_row_fast_smem(), stream>>>(
-      reinterpret_cast<const float2*>(in), reinterpret_cast<float2*>(save),
-      reinterpret_cast<float2*>(out), reinterpret_cast<const float2*>(tables),
-      reinterpret_cast<const float4*>(tw4), a);
-  return cudaGetLastError();
 }
 
 bool ifrk_fast_col(const IfrkColArgs& a) {

@@ -35,6 +35,18 @@ struct IfrkRowArgs {
 };
 
 
+// The separable Lawson factors of a one-component field for a list of stage times: table [tau]
+// [member][nx + ny], exp(i rate tau kx^2) / (nx ny) then exp(i rate tau ky^2), formed in FP64.
+constexpr int kIfrkMaxTaus = 32;
+struct LawsonTaus {
+  int count;
+  double tau[kIfrkMaxTaus];
+};
+cudaError_t launch_lawson_tables(float* tables, const double* rates, const LawsonTaus& taus, int members,
+                                 int nx, int ny, double dx, double dy, cudaStream_t stream);
+cudaError_t launch_lawson_tables(double* tables, const double* rates, const LawsonTaus& taus, int members,
+                                 int nx, int ny, double dx, double dy, cudaStream_t stream);
+
 // Per-member constants of the two-component Lawson factor (polarism/dispersion.py:34-83).
 struct SpinorConst {
   double rate;      // hbar / 2m: E(k) / hbar = rate k^2
@@ -88,5 +100,19 @@ cudaError_t launch_ifrk_col(T* psi, const T* n0, T* dn_out, T* n_out, const T* p
 
 template <typename T>
 cudaError_t configure_ifrk_kernels(size_t max_smem);
+
+// The FP32 passes on register-resident transforms (ifrk_reg.cu; axes for which reg_fft_size holds,
+// tab as launch_row_reg): attribute set-up for a grid, column panels a member, launches.
+cudaError_t configure_ifrk_reg(int nx, int ny, int comps);
+int ifrk_reg_panels(int nx, int ny, int comps, int members, int sm_count);
+cudaError_t launch_ifrk_row_reg(const float* in, float* save, float* out, const float* tables,
+                                const float* tab, const IfrkRowArgs& a, int sm_count,
+                                cudaStream_t stream);
+cudaError_t launch_ifrk_col_reg(float* psi, const float* n0, float* dn_out, float* n_out,
+                                const float* psi_start, const float* psi_new, const float* pump,
+                                const float* potential, const float* tab,
+                                const SplitConst<float>* consts, const float* scales,
+                                const unsigned long long* step_base, double* partials,
+                                const IfrkColArgs& a, int sm_count, cudaStream_t stream);
 
 }  // namespace pg

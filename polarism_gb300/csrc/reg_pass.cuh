@@ -8,6 +8,16 @@
 namespace pg {
 namespace {
 
+// The element `bytes` past a block-uniform base.
+template <typename E>
+__device__ __forceinline__ const E& at_offset(const E* base, unsigned bytes) {
+  return *reinterpret_cast<const E*>(reinterpret_cast<const char*>(base) + bytes);
+}
+template <typename E>
+__device__ __forceinline__ E& at_offset(E* base, unsigned bytes) {
+  return *reinterpret_cast<E*>(reinterpret_cast<char*>(base) + bytes);
+}
+
 // Barrier over the threads of one transform (or of a row's transforms): within a warp, or a named
 // barrier of `count` threads.
 template <bool WARP>
@@ -54,15 +64,13 @@ struct ColShape {
   static constexpr int SLOTS = RegFft<N, V>::SLOTS;
   static constexpr int REGS = sizeof(T) == 4 ? 64 : 128;  // a thread
   static constexpr int LIMIT = sizeof(T) == 4 ? 1024 : 512;
-  // 64-byte row segments (8 FP32 columns, 4 FP64), fewer where the block would be too large.
-  static constexpr int WANT = sizeof(T) == 4 ? 8 : 4;
-  static constexpr int cap(int want, int limit) {
+  // 64-byte row segments (8 FP32 columns, 4 FP64) while the block stays within LIMIT threads.
+  static constexpr int cap(int want) {
     int c = want;
-    while (c > 1 && c * M * COMPS > limit) c /= 2;
+    while (c > 1 && c * M * COMPS > LIMIT) c /= 2;
     return c;
   }
-  // Prefer blocks of half the register file or less, so that two share an SM.
-  static constexpr int MAX_COLS = cap(WANT, LIMIT / 2) >= WANT / 2 ? cap(WANT, LIMIT / 2) : cap(WANT, LIMIT);
+  static constexpr int MAX_COLS = cap(sizeof(T) == 4 ? 8 : 4);
   static constexpr int MAX_THREADS = MAX_COLS * M * COMPS < 32 ? 32 : MAX_COLS * M * COMPS;
   static constexpr int MIN_BLOCKS = 65536 / (REGS * (MAX_THREADS < 128 ? 128 : MAX_THREADS));
 };
@@ -73,10 +81,23 @@ int col_shape_cols(int nx, int members, int sm_count) {
   int cols = std::min(S::MAX_COLS, nx);
   const int least = sizeof(T) == 4 ? 2 : 1;
   while (cols > least && cols / 2 * S::M * COMPS >= 32 &&
-         static_cast<long long>(nx / cols) * members < 2LL * sm_count)
+         5LL * (nx / cols) * members < 4LL * sm_count)
     cols /= 2;
   return cols;
 }
+
+// A switch over the sizes of the passes: X(N, V) for n points (V as reg_fft_vals).
+#define PG_REG_SIZES(n, X) \
+  switch (n) {             \
+    case 64: X(64, 8);     \
+    case 128: X(128, 8);   \
+    case 256: X(256, 8);   \
+    case 512: X(512, 8);   \
+    case 1024: X(1024, 16); \
+    case 2048: X(2048, 16); \
+    case 4096: X(4096, 16); \
+    default: break;        \
+  }
 
 inline int log2_of(int n) {
   int l = 0;

@@ -68,7 +68,7 @@ struct pg_solver {
   void* tw_x = nullptr;       // exp(-2 pi i k / nx), k < nx
   void* tw_y = nullptr;
   void* prop = nullptr;       // [table][member][nx + ny] propagator factors
-  void* tw4 = nullptr;        // FP32 1024-point four-step factors W_1024^{n2 k1} (split_fast.cu)
+  void* tw4 = nullptr;        // FP32 factors W_1024^{n2 k1} of the 1024-site IFRK column pass
   void* reg_x = nullptr;      // W_n^{t k} tables of the register-resident passes (split_reg.cuh),
   void* reg_y = nullptr;      // rows and columns; null where the size has no such pass
   void* split_consts = nullptr;

@@ -97,30 +97,22 @@ cudaError_t launch_col_reg(float* data, float* res, const float* pump, const flo
                            const float* tab, const SplitConst<float>* consts, const float* scales,
                            const unsigned long long* step_base, const ColPassArgs& a, int sm_count, cudaStream_t stream);
 
-// Register-resident four-step IFRK passes for FP32 rows / columns of 1024 sites (split_fast.cu):
-// whether they apply, their W_1024^{n2 k1} table (1024 float4: rounded value, remainder) and
-// attribute set-up.
-bool split_fast_row(int nx, int ny);
-bool split_fast_col(int nx, int ny);
-void split_fast_twiddles(float* out);
-cudaError_t configure_split_fast();
-
-// The IFRK row pass on the same transforms (FP32, one component, rows of 1024 sites): whether
-// it applies and its launch (arguments as launch_ifrk_row; tw4 as above).
+// The IFRK column pass for FP32 columns of 1024 sites on 32-value transforms (ifrk_col_fast.cu;
+// one component, one single reservoir, one laser): whether a grid has it and whether it takes a
+// launch, its W_1024^{n2 k1} table (1024 float4: rounded value, remainder), attribute set-up and
+// launch.
 struct IfrkRowArgs;
 struct IfrkColArgs;
-bool ifrk_fast_row(const IfrkRowArgs& a);
-// The IFRK column pass likewise (one component, columns of 1024 sites, eight-column panels):
-// the forward-only pass, and stages and step ends with one single reservoir and one laser.
+bool ifrk_col_fast_size(int nx, int ny);
 bool ifrk_fast_col(const IfrkColArgs& a);
+void ifrk_col_fast_twiddles(float* out);
+cudaError_t configure_ifrk_col_fast();
 cudaError_t launch_ifrk_col_fast(float* psi, const float* n0, float* dn_out, float* n_out,
                                  const float* psi_start, const float* psi_new, const float* pump,
                                  const float* potential, const float* tw4,
                                  const SplitConst<float>* consts, const float* scales,
                                  const unsigned long long* step_base, const IfrkColArgs& a,
                                  cudaStream_t stream);
-cudaError_t launch_ifrk_row_fast(const float* in, float* save, float* out, const float* tables,
-                                 const float* tw4, const IfrkRowArgs& a, cudaStream_t stream);
 
 // Complex values one thread stages per FFT pass: blocks need N * C <= this * threads.
 int split_max_vals(bool is_double);

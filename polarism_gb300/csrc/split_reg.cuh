@@ -162,19 +162,6 @@ __global__ void __launch_bounds__(ColShape<T, N, V, 1>::MAX_THREADS, ColShape<T,
   for (int m = 0; m < V; ++m) d[static_cast<long long>(t + M * m) * nx] = v[m];
 }
 
-// X(N, V) for the pass of n points (V as reg_fft_vals).
-#define PG_REG_SIZES(n, X)                   \
-  switch (n) {                               \
-    case 64: X(64, 8);                       \
-    case 128: X(128, 8);                     \
-    case 256: X(256, 8);                     \
-    case 512: X(512, 8);                     \
-    case 1024: X(1024, 16);                  \
-    case 2048: X(2048, 16);                  \
-    case 4096: X(4096, 16);                  \
-    default: return cudaErrorInvalidValue;   \
-  }
-
 template <typename T>
 cudaError_t configure_row_reg(int nx) {
 #define PG_X(N, V)                                                                                     \
@@ -182,6 +169,7 @@ cudaError_t configure_row_reg(int nx) {
                               static_cast<int>(RowShape<N, V, 1>::MAX_THREADS / RowShape<N, V, 1>::M * \
                                                RowShape<N, V, 1>::STRIDE * 2 * sizeof(T)))
   PG_REG_SIZES(nx, PG_X)
+  return cudaErrorInvalidValue;
 #undef PG_X
 }
 
@@ -192,6 +180,7 @@ cudaError_t configure_col_reg(int ny) {
                               static_cast<int>(ColShape<T, N, V, 1>::MAX_COLS *                     \
                                                ColShape<T, N, V, 1>::SLOTS * 2 * sizeof(T)))
   PG_REG_SIZES(ny, PG_X)
+  return cudaErrorInvalidValue;
 #undef PG_X
 }
 
@@ -209,6 +198,7 @@ cudaError_t launch_row_reg_t(T* data, const T* tab, const T* px, const T* py, Ro
     return cudaGetLastError();                                                                     \
   }
   PG_REG_SIZES(a.nx, PG_X)
+  return cudaErrorInvalidValue;
 #undef PG_X
 }
 
@@ -229,6 +219,7 @@ cudaError_t launch_col_reg_t(T* data, T* res, const T* pump, const T* potential,
     return cudaGetLastError();                                                                        \
   }
   PG_REG_SIZES(a.ny, PG_X)
+  return cudaErrorInvalidValue;
 #undef PG_X
 }
 
