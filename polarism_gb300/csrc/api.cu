@@ -196,19 +196,20 @@ bool use_quad(const pg_solver* s, const pg::WideGeom& w) {
          pg::quad_rk4_supported(s->cfg.nx, s->cfg.ny);
 }
 
-// The tile kernel steps every FP64 grid unless the caller chose the streaming kernel or its
-// geometry: measured without / with Wigner noise, us a step, streaming kernel -> tile kernel:
-// 92.6 -> 11.4 / 141 -> 14.7 at 128^2, 179 -> 24.4 / 269 -> 35.9 at 256^2, 208 -> 78 / 314 -> 123
-// at 512^2, 310 -> 268 / 495 -> 426 at 1024^2.
-bool use_tile(const pg_solver* s) {
-  return s->rk4_kernel != 1 && !s->geom_set && s->cfg.precision == PG_DOUBLE;
+// The kernel of a step: the caller's choice (pg_rk4_set_kernel, pg_rk4_set_geometry) or the
+// automatic one.
+pg::RK4Route route(const pg_solver* s) {
+  if (s->rk4_kernel == 1 || (s->rk4_kernel == 0 && s->geom_set && !use_wide(s))) return pg::RK4Route::kStream;
+  if (s->rk4_kernel >= 2) return pg::RK4Route::kWide;
+  return s->route;
 }
 
 // Launch one RK4 step reading buffers of parity `from`; step_offset indexes the chunk scales.
 cudaError_t launch_step(pg_solver* s, int from, int step_offset) {
   const int to = 1 - from;
   const pg::RK4Features f = features(s);
-  if (use_wide(s)) {
+  const pg::RK4Route kind = route(s);
+  if (kind == pg::RK4Route::kWide) {
     pg::WideGeom w{};
     w.nx = s->cfg.nx;
     w.ny = s->cfg.ny;
@@ -241,18 +242,43 @@ cudaError_t launch_step(pg_solver* s, int from, int step_offset) {
                                static_cast<const float*>(s->scales), s->step_base, step_offset,
                                static_cast<float>(s->cfg.dt), s->noise, w, s->err_flag, s->stream);
   }
+  if (kind == pg::RK4Route::kWindow) {
+    pg::WindowGeom w = s->window;
+    w.pump_stride = s->cfg.pump_per_member ? s->plane : 0;
+    w.pump_terms = f.pump_terms;
+    w.pump_term_stride = s->pump_term_stride;
+    w.halt = s->halt;
+    w.pot = static_cast<const float*>(s->potential);
+    w.pot_stride = s->cfg.potential_per_member ? s->plane : 0;
+    w.pot_kind = f.potential;
+    w.relax = f.relax;
+    return pg::launch_rk4_window(static_cast<const float*>(s->psi[from]), static_cast<const float*>(s->res[from]),
+                                 static_cast<const float*>(s->pump), static_cast<float*>(s->psi[to]),
+                                 static_cast<float*>(s->res[to]),
+                                 static_cast<const pg::RhsConst<float>*>(s->consts),
+                                 static_cast<const float*>(s->scales), s->step_base, step_offset,
+                                 static_cast<float>(s->cfg.dt), s->noise, w, s->err_flag, s->stream);
+  }
   pg::RK4Geom g = s->geom;
   g.pump_stride = s->cfg.pump_per_member ? s->plane : 0;
   g.pot_stride = s->cfg.potential_per_member ? s->plane : 0;
   g.halt = s->halt;
   g.pump_term_stride = s->pump_term_stride;
-  if (use_tile(s))
-    return pg::launch_rk4_tile_f64(
-        s->tile_shape, static_cast<const double*>(s->psi[from]), static_cast<const double*>(s->res[from]),
-        static_cast<const double*>(s->pump), static_cast<const double*>(s->potential),
-        static_cast<double*>(s->psi[to]), static_cast<double*>(s->res[to]),
-        static_cast<const pg::RhsConst<double>*>(s->consts), static_cast<const double*>(s->scales),
-        s->step_base, step_offset, s->cfg.dt, s->noise, g, f, s->stream);
+  if (kind == pg::RK4Route::kTile) {
+    if (s->cfg.precision == PG_DOUBLE)
+      return pg::launch_rk4_tile_f64(
+          s->tile_shape, static_cast<const double*>(s->psi[from]), static_cast<const double*>(s->res[from]),
+          static_cast<const double*>(s->pump), static_cast<const double*>(s->potential),
+          static_cast<double*>(s->psi[to]), static_cast<double*>(s->res[to]),
+          static_cast<const pg::RhsConst<double>*>(s->consts), static_cast<const double*>(s->scales),
+          s->step_base, step_offset, s->cfg.dt, s->noise, g, f, s->stream);
+    return pg::launch_rk4_tile_f32(
+        s->tile_shape, static_cast<const float*>(s->psi[from]), static_cast<const float*>(s->res[from]),
+        static_cast<const float*>(s->pump), static_cast<const float*>(s->potential),
+        static_cast<float*>(s->psi[to]), static_cast<float*>(s->res[to]),
+        static_cast<const pg::RhsConst<float>*>(s->consts), static_cast<const float*>(s->scales),
+        s->step_base, step_offset, static_cast<float>(s->cfg.dt), s->noise, g, f, s->stream);
+  }
   if (s->cfg.precision == PG_DOUBLE) {
     return pg::launch_rk4_step<double>(
         static_cast<const double*>(s->psi[from]), static_cast<const double*>(s->res[from]),
@@ -440,8 +466,16 @@ int pg_create(const pg_config* cfg, const pg_physics* physics, pg_solver** out) 
       return fail(e, "staging event");
   }
   pg::choose_rk4_geometry(cfg->nx, cfg->ny, cfg->members, cfg->precision, s->sm_count, &s->geom);
-  if (cfg->precision == PG_DOUBLE)
+  if (cfg->precision == PG_DOUBLE) {
+    // The tile kernel steps every FP64 grid: measured without / with Wigner noise, us a step,
+    // streaming kernel -> tile kernel: 92.6 -> 11.4 / 141 -> 14.7 at 128^2, 179 -> 24.4 / 269 ->
+    // 35.9 at 256^2, 208 -> 78 / 314 -> 123 at 512^2, 310 -> 268 / 495 -> 426 at 1024^2.
+    s->route = pg::RK4Route::kTile;
     s->tile_shape = pg::choose_rk4_tile_f64(cfg->nx, cfg->ny, cfg->members, s->sm_count);
+  } else {
+    s->route = pg::choose_rk4_route(cfg->nx, cfg->ny, cfg->members, s->sm_count, features(s), s->geom,
+                                    &s->window, &s->tile_shape);
+  }
   int rc = upload_consts(s);
   if (rc != PG_OK) {
     release(s);

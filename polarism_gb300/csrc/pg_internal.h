@@ -105,6 +105,13 @@ cudaError_t launch_rk4_tile_f64(int shape, const double* psi_in, const double* n
                                 bool noise, const RK4Geom& g, const RK4Features& f,
                                 cudaStream_t stream);
 
+cudaError_t launch_rk4_tile_f32(int shape, const float* psi_in, const float* n_in, const float* pump,
+                                const float* potential, float* psi_out, float* n_out,
+                                const RhsConst<float>* consts, const float* scales,
+                                const unsigned long long* step_base, int step_offset, float dt,
+                                bool noise, const RK4Geom& g, const RK4Features& f,
+                                cudaStream_t stream);
+
 // Choose the tile width / strip height for a grid (deterministic heuristic,
 // overridable through the autotuner table).
 void choose_rk4_geometry(int nx, int ny, int members, int precision, int sm_count,
@@ -112,5 +119,12 @@ void choose_rk4_geometry(int nx, int ny, int members, int precision, int sm_coun
 
 int philox_words_device(const uint32_t* counters, uint64_t key, uint32_t* out, int64_t n,
                         cudaStream_t stream);
+
+struct WindowGeom;
+// The kernel an FP32 grid is stepped with when the caller leaves the choice (rk4_plan.cu); fills the
+// window's geometry or the tile's shape for it.
+enum class RK4Route { kStream, kWide, kWindow, kTile };
+RK4Route choose_rk4_route(int nx, int ny, int members, int sm_count, const RK4Features& f,
+                          const RK4Geom& stream, WindowGeom* window, int* tile);
 
 }  // namespace pg

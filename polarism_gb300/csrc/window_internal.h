@@ -1,0 +1,50 @@
+// Internal declarations of the FP32 RK4 window kernel (rk4_window.cuh).
+#pragma once
+#include <cuda_runtime.h>
+
+#include "pg_internal.h"
+
+namespace pg {
+
+struct WindowGeom {
+  int nx, ny, members;
+  int bands;               // windows a row; 1: the row closes on itself
+  int band_w;              // columns a band writes (even when bands > 1)
+  int wmax;                // window capacity: 256, 320, 512 or 1024 columns
+  int blocks;              // persistent grid
+  long long pump_stride;   // 0: shared envelope; nx*ny: one per member
+  int pump_terms;
+  long long pump_term_stride;
+  const int* halt;
+  const float* pot;        // potential: none, real or complex (pot_kind 0, 1, 2)
+  long long pot_stride;
+  int pot_kind;
+  int relax;
+};
+
+double row_iterations(long long units, int ny, long long blocks);
+long long row_blocks(long long units, int ny, long long slots);
+// Picks bands, band_w, wmax and blocks for a grid; the modelled time in us.
+double choose_rk4_window(int nx, int ny, int members, int sm_count, WindowGeom* g);
+cudaError_t launch_rk4_window(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
+                              float* n_out, const RhsConst<float>* consts, const float* scales,
+                              const unsigned long long* step_base, int step_offset, float dt, bool noise,
+                              const WindowGeom& g, int* err_flag, cudaStream_t stream);
+cudaError_t launch_rk4_window_256(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
+                              float* n_out, const RhsConst<float>* consts, const float* scales,
+                              const unsigned long long* step_base, int step_offset, float dt, bool noise,
+                              const WindowGeom& g, int* err_flag, cudaStream_t stream);
+cudaError_t launch_rk4_window_320(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
+                              float* n_out, const RhsConst<float>* consts, const float* scales,
+                              const unsigned long long* step_base, int step_offset, float dt, bool noise,
+                              const WindowGeom& g, int* err_flag, cudaStream_t stream);
+cudaError_t launch_rk4_window_512(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
+                              float* n_out, const RhsConst<float>* consts, const float* scales,
+                              const unsigned long long* step_base, int step_offset, float dt, bool noise,
+                              const WindowGeom& g, int* err_flag, cudaStream_t stream);
+cudaError_t launch_rk4_window_1024(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
+                              float* n_out, const RhsConst<float>* consts, const float* scales,
+                              const unsigned long long* step_base, int step_offset, float dt, bool noise,
+                              const WindowGeom& g, int* err_flag, cudaStream_t stream);
+
+}  // namespace pg
