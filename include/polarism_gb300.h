@@ -335,8 +335,8 @@ int pg_sweep_set_noise(pg_sweep* w, const uint64_t* seeds, const double* gamma,
                        const double* scattering, const double* strength);
 /* Tile shape of the persistent launch: `lanes` columns per block (512 or 1024; a block stacks
  * lanes / nx strips of equally wide members side by side, so every member needs
- * lanes / 8 <= nx <= lanes) and `strip_rows` rows per work item (>= 8).  The choice changes
- * speed only, never results.  pg_sweep_get_tiling also reports the work items and the grid. */
+ * lanes / 8 <= nx <= lanes) and at most `strip_rows` rows per work item (>= 8; the strips are cut
+ * shorter where that fills the last wave of blocks).  The choice changes speed only, never results.  pg_sweep_get_tiling also reports the work items and the grid. */
 int pg_sweep_set_tiling(pg_sweep* w, int32_t lanes, int32_t strip_rows);
 int pg_sweep_get_tiling(pg_sweep* w, int32_t* lanes, int32_t* strip_rows, int32_t* items,
                         int32_t* blocks);

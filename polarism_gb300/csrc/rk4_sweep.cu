@@ -546,17 +546,66 @@ int lanes_blocks_per_sm(int lanes, bool noise) {
   return lanes == 1024 ? pg::blocks_per_sm<1024>(noise) : pg::blocks_per_sm<512>(noise);
 }
 
+// Height of a member's strips when none may have more than `rows` rows: as many strips as that
+// takes, all alike but the last.
+int strip_height(int ny, int rows) {
+  const int strips = (ny + rows - 1) / rows;
+  return (ny + strips - 1) / strips;
+}
+
+// Work items of the active members with strips of at most `rows` rows.
+long long count_items(const pg_sweep* w, int lanes, int rows) {
+  std::map<std::pair<int, int>, long long> strips;  // (nx, h) -> strips
+  for (int m = 0; m < w->members; ++m) {
+    if (!w->active[m]) continue;
+    const int ny = w->grids[m].ny, h = strip_height(ny, rows);
+    strips[{w->grids[m].nx, h}] += ny / h;
+    if (ny % h) strips[{w->grids[m].nx, ny % h}] += 1;
+  }
+  long long items = 0;
+  for (const auto& kv : strips) {
+    const long long per_item = lanes / kv.first.first;
+    items += (kv.second + per_item - 1) / per_item;
+  }
+  return items;
+}
+
+// The shortest strips that still make no more items than `strip_rows` does, rounded up to whole
+// waves of resident blocks.  With strips of exactly `strip_rows` rows, 16 members each of 128^2,
+// 256^2 and 512^2 are 168 items of 64 rows or 336 of 32 for 304 resident blocks: 57.6 us a step at the
+// best power of two, 45.1 with 280 items of 40 rows (with noise 77.6 and 65.0).
+// Multiples of 8 rows: the kernel works in whole turns of its ring (ending an item within a turn costs
+// every iteration 15 to 25 %, the unrolled turn being one schedule no longer).
+int fitted_rows(const pg_sweep* w, int lanes, int strip_rows) {
+  const long long resident = static_cast<long long>(lanes_blocks_per_sm(lanes, true)) * w->sm_count;
+  int max_ny = 8;
+  for (const auto& g : w->grids) max_ny = std::max(max_ny, g.ny);
+  strip_rows = std::min(strip_rows, max_ny);
+  const long long items = count_items(w, lanes, strip_rows);
+  const long long limit = (items + resident - 1) / resident * resident;
+  int lo = 1, best = (strip_rows + 7) / 8;  // bisection: the count all but falls with the height
+  while (lo < best) {
+    const int mid = (lo + best) / 2;
+    if (count_items(w, lanes, 8 * mid) <= limit)
+      best = mid;
+    else
+      lo = mid + 1;
+  }
+  return 8 * best;
+}
+
 // Rebuild the item list for (lanes, strip_rows) over the active members.  Strips of equal
 // width and height are packed lanes / W to an item; items are ordered tallest first so the
 // strided walk of the persistent blocks spreads the heavy ones.
 int build_items(pg_sweep* w, int lanes, int strip_rows) {
   std::map<std::pair<int, int>, std::vector<pg::SweepStrip>> groups;  // (wl2, h) -> strips
+  const int rows = fitted_rows(w, lanes, strip_rows);
   for (int m = 0; m < w->members; ++m) {
     if (!w->active[m]) continue;
     const int nx = w->grids[m].nx, ny = w->grids[m].ny;
-    const int wl2 = ilog2(nx);
-    for (int y0 = 0; y0 < ny; y0 += strip_rows)
-      groups[{wl2, std::min(strip_rows, ny - y0)}].push_back(pg::SweepStrip{m, y0});
+    const int wl2 = ilog2(nx), h = strip_height(ny, rows);
+    for (int y0 = 0; y0 < ny; y0 += h)
+      groups[{wl2, std::min(h, ny - y0)}].push_back(pg::SweepStrip{m, y0});
   }
   std::vector<SweepItem> items;
   for (auto& kv : groups) {
@@ -608,7 +657,7 @@ int check_tiling(const pg_sweep* w, int lanes, int strip_rows) {
 }
 
 // Default tiling before any measurement: the narrowest lanes that hold every member, and
-// the strip height whose modelled time (waves of equal items x rows per item incl. the
+// the strip height whose modelled time (waves of equal items x iterations per item incl. the
 // 8-row pipeline fill) is smallest.
 void default_tiling(const pg_sweep* w, int* lanes, int* strip_rows) {
   int max_nx = 0, max_ny = 0;
@@ -618,29 +667,15 @@ void default_tiling(const pg_sweep* w, int* lanes, int* strip_rows) {
   }
   *lanes = max_nx <= 512 ? 512 : 1024;
   const long long resident = static_cast<long long>(lanes_blocks_per_sm(*lanes, true)) * w->sm_count;
-  double best = 1e300;
-  int best_h = 8;
+  long long best = -1;
   for (int h = 8; h <= std::max(8, max_ny); h *= 2) {
-    std::map<std::pair<int, int>, long long> strips;
-    for (const auto& g : w->grids)
-      for (int y0 = 0; y0 < g.ny; y0 += h) strips[{g.nx, std::min(h, g.ny - y0)}] += 1;
-    double rows = 0.0;
-    long long items = 0;
-    for (const auto& kv : strips) {
-      const long long per = *lanes / kv.first.first;
-      const long long n = (kv.second + per - 1) / per;
-      items += n;
-      rows += static_cast<double>(n) * (((kv.first.second + 8 + 7) / 8) * 8);
-    }
-    const double waves = std::ceil(static_cast<double>(items) / static_cast<double>(resident));
-    const double per_item = rows / std::max<long long>(1, items);
-    const double cost = waves * per_item;
-    if (cost < best) {
+    const int rows = fitted_rows(w, *lanes, h);
+    const long long cost = (count_items(w, *lanes, rows) + resident - 1) / resident * ((rows + 15) / 8);
+    if (best < 0 || cost < best) {
       best = cost;
-      best_h = h;
+      *strip_rows = h;
     }
   }
-  *strip_rows = best_h;
 }
 
 cudaError_t launch_sweep_step(pg_sweep* w, int from, int step_offset) {

@@ -260,7 +260,8 @@ def _cache_key(engine: SweepEngine, noise: bool) -> str:
     sizes = {}
     for nx, ny, _, _ in engine.grids:
         sizes[f"{ny}x{nx}"] = sizes.get(f"{ny}x{nx}", 0) + 1
-    return json.dumps([device, sorted(sizes.items()), bool(noise)])
+    # "cut": timings taken with strips of exactly strip_rows rows ranked the shapes differently.
+    return json.dumps([device, sorted(sizes.items()), bool(noise), "cut"])
 
 
 def _write_cache(path: Path, cache: dict) -> None:
