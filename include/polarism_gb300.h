@@ -420,6 +420,34 @@ int pg_fno_mode_mix(const float* y, const void* wre, const void* wim, float* out
 int pg_fno_mode_mix_backward(const float* y, const float* dout, const void* wre, const void* wim, float* dy,
                              float* dwre, float* dwim, int32_t B, int32_t cin, int32_t cout, int32_t modes,
                              void* stream);
+/* The same with BF16 results (the next GEMM's operand), FP32 ones, or both. */
+int pg_fno_mode_mix_bf16(const float* y, const void* wre, const void* wim, float* out, void* out_bf16, int32_t B,
+                         int32_t cin, int32_t cout, int32_t modes, void* stream);
+int pg_fno_mode_mix_backward_bf16(const float* y, const float* dout, const void* wre, const void* wim, float* dy,
+                                  void* dy_bf16, float* dwre, float* dwim, int32_t B, int32_t cin, int32_t cout,
+                                  int32_t modes, void* stream);
+/* Fused passes of the operator (csrc/fno_fused.cu).  pg_fno_fused: 1 when they serve a network of up to
+ * max_channels channels on n x n sites with `modes` modes (n a multiple of 8, modes of 4, at most 128
+ * channels, tcgen05 as the engine); the general calls above serve every network, with the same results.
+ *
+ * pg_fno_layer: x[b, co, p] = sum_k w[co, k] v[b, k, p] (+ sum_q z[b, co, y, q] table[q, x]) (+ bias[co]);
+ * mode 0 writes x, mode 1 x to u and GELU(x) to out_bf16, mode 2 x GELU'(pre) to both.  w is
+ * [cout][cin], or [cin][cout] when w_transposed; z is [B][cout][n][modes2] and table [modes2][n], or
+ * [n][modes2] when table_rows (modes2 = 0: no spectral term); u (FP32) and out_bf16 may be NULL.
+ * pg_fno_outer: parts[b, s] = g[b] x[b]^T over slice s of the plane (plane / slices a multiple of 8).
+ * pg_fno_dft_y: G s, or G^H s when inverse, for `batch` complex matrices with columns re | im.
+ * pg_fno_dft_x: out = v table for `rows` rows of n values; table [n][2 modes], or [2 modes][n] when
+ * table_rows. */
+int pg_fno_fused(int32_t n, int32_t modes, int32_t max_channels, int32_t* fused);
+int pg_fno_layer(const void* w, int32_t w_transposed, const void* v, const void* z, const void* table,
+                 int32_t table_rows, const float* bias, const float* pre, float* u, void* out_bf16,
+                 int32_t B, int32_t cin, int32_t cout, int32_t n, int32_t modes2, int32_t mode, void* stream);
+int pg_fno_outer(const void* g, const void* x, float* parts, int32_t B, int32_t cout, int32_t cin, int64_t plane,
+                 int32_t slices, void* stream);
+int pg_fno_dft_y(const void* gre, const void* gim, const void* s, float* out, void* out_bf16, int32_t batch,
+                 int32_t n, int32_t modes, int32_t inverse, void* stream);
+int pg_fno_dft_x(const void* v, const void* table, int32_t table_rows, void* out_bf16, int64_t rows, int32_t n,
+                 int32_t modes, void* stream);
 /* Adam on FP32 weights (bias-corrected, optional L2 decay), refreshing the BF16 copy. */
 int pg_fno_adam(float* w, const float* g, float* m1, float* m2, void* w_bf16, int64_t n, float lr,
                 float beta1, float beta2, float eps, int64_t step, float decay, void* stream);

@@ -139,6 +139,15 @@ SIGNATURES = {
     "pg_fno_mode_mix": (C.c_int, [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
     "pg_fno_mode_mix_backward": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32,
                                            _i32, _vp]),
+    "pg_fno_mode_mix_bf16": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
+    "pg_fno_mode_mix_backward_bf16": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32,
+                                                _i32, _i32, _vp]),
+    "pg_fno_fused": (C.c_int, [_i32, _i32, _i32, C.POINTER(_i32)]),
+    "pg_fno_layer": (C.c_int, [_vp, _i32, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _i32, _i32, _i32,
+                               _i32, _i32, _i32, _vp]),
+    "pg_fno_outer": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _i64, _i32, _vp]),
+    "pg_fno_dft_y": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
+    "pg_fno_dft_x": (C.c_int, [_vp, _vp, _i32, _vp, _i64, _i32, _i32, _vp]),
     "pg_fno_adam": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _i64, C.c_float, C.c_float, C.c_float,
                               C.c_float, _i64, C.c_float, _vp]),
     "pg_fno_mse": (C.c_int, [_vp, _vp, _vp, _i32, _i64, _vp, _vp, _vp, _i32, _i64, C.c_float,

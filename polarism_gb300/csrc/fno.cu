@@ -13,6 +13,8 @@
 #include <cstdint>
 
 #include "pg_internal.h"
+#include "fno_internal.h"
+#include "tc05.cuh"
 #include "tma.cuh"
 
 namespace pg {
@@ -170,34 +172,9 @@ constexpr int kTcSmemB = kTcN * kTcK * 2;                // 8 KB
 constexpr int kTcSmem = 28 * 1024;
 constexpr int kTcWaitLimit = 200000;
 
-__device__ __forceinline__ uint64_t tc_smem_desc(uint32_t addr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((addr & 0x3FFFF) >> 4);            // start address
-  d |= static_cast<uint64_t>(128 >> 4) << 16;                    // leading byte offset (K)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;                   // stride byte offset (8 rows)
-  d |= static_cast<uint64_t>(1) << 46;                           // descriptor version
-  return d;                                                      // base offset 0, no swizzle
-}
-
 // kind::f16 instruction descriptor: D = F32, A = B = BF16, both K-major, N = 64, M = 128.
 constexpr uint32_t kTcIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kTcN >> 3) << 17) |
                               (static_cast<uint32_t>(kTcM >> 4) << 24);
-
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, int accumulate) {
-  asm volatile(
-      "{\n"
-      " .reg .pred p;\n"
-      " setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
-               : "memory");
-}
 
 // One K slab of an operand into the canonical K-major layout: ROWS rows (M or N) x 64 k.
 // kmajor: element (r, k) at X[r * ld + k], else at X[k * ld + r].  With vec, rows start on
@@ -328,7 +305,7 @@ __global__ void __launch_bounds__(128, 1) gemm_bf16_tc05_kernel(const GemmArgs g
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int s = 0; s < kTcK / 16; ++s)
-        tc_mma(tmem, tc_smem_desc(a_base + 256 * s), tc_smem_desc(b_base + 256 * s), kTcIdesc,
+        tc_mma(tmem, tc_smem_desc(a_base + 256 * s, 128, 1024), tc_smem_desc(b_base + 256 * s, 128, 1024), kTcIdesc,
                (slab > 0 || s > 0) ? 1 : 0);
       tc_commit(smem_u32(mbar));
     }
@@ -397,6 +374,7 @@ __global__ void sum_slices_kernel(const float* __restrict__ parts, float* __rest
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float s = accumulate ? out[i] : 0.f;
+#pragma unroll 32
     for (int c = 0; c < count; ++c) s += parts[static_cast<long long>(c) * n + i];
     out[i] = s;
   }
@@ -406,17 +384,6 @@ __global__ void to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __res
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x)
     y[i] = __float2bfloat16_rn(x[i]);
-}
-
-constexpr float kGeluC = 0.7978845608028654f;  // sqrt(2 / pi)
-
-__device__ __forceinline__ float gelu_f(float x) {
-  return 0.5f * x * (1.f + tanhf(kGeluC * (x + 0.044715f * x * x * x)));
-}
-
-__device__ __forceinline__ float gelu_grad_f(float x) {
-  const float t = tanhf(kGeluC * (x + 0.044715f * x * x * x));
-  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * kGeluC * (1.f + 3.f * 0.044715f * x * x);
 }
 
 // u[b, c, p] += bias[c]; act = gelu(u) (or u) in FP32 and, optionally, in BF16.
@@ -445,107 +412,229 @@ __global__ void gelu_back_kernel(const float* __restrict__ pre, const float* __r
   }
 }
 
-// out[c] = (accumulate ? out[c] : 0) + sum over b, p of x[b, c, p]; one block per channel.
-__global__ void channel_sum_kernel(const float* __restrict__ x, float* __restrict__ out, int B, int C,
-                                   long long plane, int accumulate) {
+// out[c] = (accumulate ? out[c] : 0) + sum over b, p of x[b, c, p]; one block per channel, thread t adding
+// the values t, t + 256, ... of each sample in turn, so that every sum has one fixed order.  Few blocks, each
+// bound by its own loads in flight: with 16-byte rows (RING) 160 KB of copies are in flight to a ring
+// in shared memory; otherwise 16 loads a thread.  8 x 32 x 256^2 values: 453 us with one load a thread
+// at a time, 163 with 4-byte copies, 44 with 16-byte ones and 16 values a thread between barriers, 27 with 32.
+constexpr int kSumChunk = 8192;  // values a ring slot
+constexpr int kSumRing = 6;
+template <bool RING>
+__global__ void __launch_bounds__(256) channel_sum_kernel(const float* __restrict__ x, float* __restrict__ out,
+                                                          int B, int C, long long plane, int accumulate) {
+  extern __shared__ __align__(16) float ring[];
   __shared__ float red[32];
-  const int c = blockIdx.x;
+  const int c = blockIdx.x, t = threadIdx.x;
   float s = 0.f;
-  for (int b = 0; b < B; ++b) {
-    const float* p = x + (static_cast<long long>(b) * C + c) * plane;
-    for (long long i = threadIdx.x; i < plane; i += blockDim.x) s += p[i];
+  if (RING) {
+    const long long per = (plane + kSumChunk - 1) / kSumChunk, total = per * B;
+    int lb = 0, lc = 0;  // sample and chunk of the next copy
+    auto copy = [&](int slot) {
+      if (lb < B) {
+        const long long p0 = static_cast<long long>(lc) * kSumChunk;
+        const float* src = x + (static_cast<long long>(lb) * C + c) * plane + p0;
+        const int n = static_cast<int>(plane - p0 < kSumChunk ? plane - p0 : kSumChunk);
+        float* dst = ring + slot * kSumChunk + 4 * t;
+        src += 4 * t;
+        if (n == kSumChunk) {
+#pragma unroll
+          for (int q = 0; q < kSumChunk / 1024; ++q) cp_async16(dst + 1024 * q, src + 1024 * q);
+        } else {
+          for (int e = 0; 4 * t + e < n; e += 1024) cp_async16(dst + e, src + e);
+        }
+        if (++lc == per) {
+          lc = 0;
+          ++lb;
+        }
+      }
+      cp_async_commit();
+    };
+    for (int g = 0; g < kSumRing - 1; ++g) copy(g);
+    int slot = 0, cc = 0;
+    for (long long g = 0; g < total; ++g) {
+      cp_async_wait<kSumRing - 2>();
+      __syncthreads();
+      copy(slot == 0 ? kSumRing - 1 : slot - 1);  // the slot read before the barrier
+      const long long p0 = static_cast<long long>(cc) * kSumChunk;
+      const float* v = ring + slot * kSumChunk + t;
+      if (plane - p0 >= kSumChunk) {
+#pragma unroll
+        for (int q = 0; q < kSumChunk / 256; ++q) s += v[q * 256];
+      } else {
+        for (int q = 0; t + q * 256 < plane - p0; ++q) s += v[q * 256];
+      }
+      cc = cc + 1 == per ? 0 : cc + 1;
+      slot = slot + 1 == kSumRing ? 0 : slot + 1;
+    }
+    cp_async_wait<0>();
+  } else {
+    for (int b = 0; b < B; ++b) {
+      const float* p = x + (static_cast<long long>(b) * C + c) * plane;
+      long long i = t;
+      for (; i + 15 * 256 < plane; i += 16 * 256) {
+        float v[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = p[i + q * 256];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) s += v[q];
+      }
+      for (; i < plane; i += 256) s += p[i];
+    }
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  if ((t & 31) == 0) red[t >> 5] = s;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    float v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.f;
+  if (t < 32) {
+    float v = t < (blockDim.x >> 5) ? red[t] : 0.f;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0) out[c] = (accumulate ? out[c] : 0.f) + v;
+    if (t == 0) out[c] = (accumulate ? out[c] : 0.f) + v;
   }
 }
 
 // Spectra are stored [b][channel][ky (2m)][kx re (m) | kx im (m)]; weights [ky][kx][in][out].
-__global__ void mode_mix_kernel(const float* __restrict__ y, const __nv_bfloat16* __restrict__ wre,
-                                const __nv_bfloat16* __restrict__ wim, float* __restrict__ out,
-                                int B, int cin, int cout, int m) {
-  const long long total = static_cast<long long>(B) * cout * 2 * m * m;
-  const int mm = 2 * m * m;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int mode = static_cast<int>(t % mm);
-    const int o = static_cast<int>((t / mm) % cout);
-    const int b = static_cast<int>(t / (static_cast<long long>(mm) * cout));
-    const int ky = mode / m, kx = mode % m;
-    float re = 0.f, im = 0.f;
-    const float* yb = y + static_cast<long long>(b) * cin * 4 * m * m + ky * 2 * m;
-    const long long wbase = (static_cast<long long>(ky) * m + kx) * cin * cout + o;
-    for (int i = 0; i < cin; ++i) {
-      const float a = yb[static_cast<long long>(i) * 4 * m * m + kx];
-      const float c = yb[static_cast<long long>(i) * 4 * m * m + m + kx];
-      const float r = __bfloat162float(wre[wbase + static_cast<long long>(i) * cout]);
-      const float s = __bfloat162float(wim[wbase + static_cast<long long>(i) * cout]);
-      re += a * r - c * s;
-      im += a * s + c * r;
-    }
-    float* ob = out + (static_cast<long long>(b) * cout + o) * 4 * m * m + ky * 2 * m;
-    ob[kx] = re;
-    ob[m + kx] = im;
+//
+// One block a mode.  A mode's spectral values lie a whole spectrum apart and its weights in one run, so the
+// block first gathers both into shared memory, every load in flight at once, and computes from there;
+// with one thread an output reading them as it went, each product waited for its own sectors.  8 x 32
+// channels, 512 modes: mixing 38 -> 12 us, its adjoints 38 -> 11 and 36 -> 9 us.
+constexpr int kMixSamples = 8;                // samples gathered at a time, at most
+constexpr size_t kMixSmem = 200 * 1024;
+
+// The fused multiply-adds are spelled out: one rounding more or less in a spectral value moves the BF16
+// rounding of the operands after it.
+struct MixStage {
+  int samples;    // gathered at a time
+  int weights;    // the mode's weights too (they fit)
+  size_t bytes;
+};
+
+MixStage mix_stage(int values_per_sample, long long weights, int B) {
+  MixStage m{};
+  const long long fit = static_cast<long long>(kMixSmem / 2) / (8LL * values_per_sample);
+  m.samples = static_cast<int>(fit < 1 ? 1 : fit < kMixSamples ? fit : kMixSamples);
+  if (m.samples > B) m.samples = B;
+  m.bytes = static_cast<size_t>(m.samples) * values_per_sample * 8;
+  m.weights = weights * 4 <= static_cast<long long>(kMixSmem / 2);
+  if (m.weights) m.bytes += static_cast<size_t>(weights) * 4;
+  return m;
+}
+
+// vals[q] = the mode's value of the q-th of `count` consecutive (sample, channel) spectra from x.
+__device__ __forceinline__ void gather_mode(float2* vals, const float* x, int count, int m, int at) {
+#pragma unroll 2
+  for (int q = threadIdx.x; q < count; q += blockDim.x) {
+    const float* src = x + static_cast<long long>(q) * (4 * m * m) + at;
+    vals[q] = make_float2(src[0], src[m]);
   }
 }
 
-// dY[b, i] = sum_o dO[b, o] conj(W[i, o]) per mode.
-__global__ void mode_mix_back_input_kernel(const float* __restrict__ dout, const __nv_bfloat16* __restrict__ wre,
-                                           const __nv_bfloat16* __restrict__ wim, float* __restrict__ dy,
-                                           int B, int cin, int cout, int m) {
-  const long long total = static_cast<long long>(B) * cin * 2 * m * m;
-  const int mm = 2 * m * m;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int mode = static_cast<int>(t % mm);
-    const int i = static_cast<int>((t / mm) % cin);
-    const int b = static_cast<int>(t / (static_cast<long long>(mm) * cin));
-    const int ky = mode / m, kx = mode % m;
-    float re = 0.f, im = 0.f;
-    const float* gb = dout + static_cast<long long>(b) * cout * 4 * m * m + ky * 2 * m;
-    const long long wbase = ((static_cast<long long>(ky) * m + kx) * cin + i) * cout;
-    for (int o = 0; o < cout; ++o) {
-      const float gr = gb[static_cast<long long>(o) * 4 * m * m + kx];
-      const float gi = gb[static_cast<long long>(o) * 4 * m * m + m + kx];
-      const float r = __bfloat162float(wre[wbase + o]);
-      const float s = __bfloat162float(wim[wbase + o]);
-      re += gr * r + gi * s;
-      im += gi * r - gr * s;
+__device__ __forceinline__ void put_mode(float* out, __nv_bfloat16* out_bf, long long at, int m, float re, float im) {
+  if (out) {
+    out[at] = re;
+    out[at + m] = im;
+  }
+  if (out_bf) {
+    out_bf[at] = __float2bfloat16_rn(re);
+    out_bf[at + m] = __float2bfloat16_rn(im);
+  }
+}
+
+// out[b, o] = sum_i y[b, i] W[i, o], or with ADJOINT dY[b, i] = sum_o dO[b, o] conj(W[i, o]); n_in and n_out
+// are the channels summed over and written.  out and out_bf: either may be null.
+template <bool ADJOINT>
+__global__ void __launch_bounds__(256)
+    mode_mix_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ wre,
+                    const __nv_bfloat16* __restrict__ wim, float* __restrict__ out, __nv_bfloat16* __restrict__ out_bf,
+                    int B, int n_in, int n_out, int m, const MixStage st) {
+  extern __shared__ float2 vals[];  // [samples][n_in], then the weights
+  const int ky = blockIdx.x / m, kx = blockIdx.x % m;
+  const int at = ky * 2 * m + kx, weights = n_in * n_out;
+  const int len = ADJOINT ? n_in : n_out;          // the weights' rows are [in][out]
+  const int pitch = st.weights ? len + 2 : len;    // staged rows start on different banks
+  const __nv_bfloat16* re_w = wre + static_cast<long long>(blockIdx.x) * weights;
+  const __nv_bfloat16* im_w = wim + static_cast<long long>(blockIdx.x) * weights;
+  if (st.weights) {
+    __nv_bfloat16* sw = reinterpret_cast<__nv_bfloat16*>(vals + st.samples * n_in);
+#pragma unroll 4
+    for (int e = threadIdx.x; e < weights; e += blockDim.x) {
+      const int d = e / len * pitch + e % len;
+      sw[d] = re_w[e];
+      sw[weights / len * pitch + d] = im_w[e];
     }
-    float* db = dy + (static_cast<long long>(b) * cin + i) * 4 * m * m + ky * 2 * m;
-    db[kx] = re;
-    db[m + kx] = im;
+    re_w = sw;
+    im_w = sw + weights / len * pitch;
+  }
+  for (int b0 = 0; b0 < B; b0 += st.samples) {
+    const int nb = min(st.samples, B - b0);
+    if (b0) __syncthreads();
+    gather_mode(vals, x + static_cast<long long>(b0) * n_in * (4 * m * m), nb * n_in, m, at);
+    __syncthreads();
+    for (int t = threadIdx.x; t < nb * n_out; t += blockDim.x) {
+      const int c = t % n_out, b = t / n_out;
+      const float2* v = vals + b * n_in;
+      float re = 0.f, im = 0.f;
+#pragma unroll 4
+      for (int k = 0; k < n_in; ++k) {
+        const int w = ADJOINT ? c * pitch + k : k * pitch + c;
+        const float r = __bfloat162float(re_w[w]), s = __bfloat162float(im_w[w]);
+        if (ADJOINT) {
+          const float gr = v[k].x, gi = v[k].y;
+          re += __fmaf_rn(gr, r, __fmul_rn(gi, s));
+          im += __fmaf_rn(gi, r, -__fmul_rn(gr, s));
+        } else {
+          const float a = v[k].x, c2 = v[k].y;
+          re += __fmaf_rn(a, r, -__fmul_rn(c2, s));
+          im += __fmaf_rn(c2, r, __fmul_rn(a, s));
+        }
+      }
+      put_mode(out, out_bf, (static_cast<long long>(b0 + b) * n_out + c) * (4 * m * m) + at, m, re, im);
+    }
   }
 }
 
 // dW[i, o] = sum_b conj(Y[b, i]) dO[b, o] per mode (overwrites).
-__global__ void mode_mix_back_weight_kernel(const float* __restrict__ y, const float* __restrict__ dout,
-                                            float* __restrict__ dwre, float* __restrict__ dwim,
-                                            int B, int cin, int cout, int m) {
-  const long long total = static_cast<long long>(2 * m) * m * cin * cout;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int o = static_cast<int>(t % cout);
-    const int i = static_cast<int>((t / cout) % cin);
-    const int mode = static_cast<int>(t / (static_cast<long long>(cout) * cin));
-    const int ky = mode / m, kx = mode % m;
-    float re = 0.f, im = 0.f;
-    for (int b = 0; b < B; ++b) {
-      const float* yb = y + (static_cast<long long>(b) * cin + i) * 4 * m * m + ky * 2 * m;
-      const float* gb = dout + (static_cast<long long>(b) * cout + o) * 4 * m * m + ky * 2 * m;
-      const float a = yb[kx], c = yb[m + kx];
-      const float gr = gb[kx], gi = gb[m + kx];
-      re += a * gr + c * gi;
-      im += a * gi - c * gr;
+__global__ void __launch_bounds__(256) mode_mix_back_weight_kernel(const float* __restrict__ y,
+                                                                   const float* __restrict__ dout,
+                                                                   float* __restrict__ dwre, float* __restrict__ dwim,
+                                                                   int B, int cin, int cout, int m, int samples) {
+  extern __shared__ float2 vals[];  // [samples][cin], [samples][cout]
+  float2* ys = vals;
+  float2* gs = vals + samples * cin;
+  const int at = static_cast<int>(blockIdx.x / m) * 2 * m + static_cast<int>(blockIdx.x % m);
+  const long long wbase = static_cast<long long>(blockIdx.x) * cin * cout;
+  for (int b0 = 0; b0 < B; b0 += samples) {
+    const int nb = min(samples, B - b0);
+    if (b0) __syncthreads();
+    gather_mode(ys, y + static_cast<long long>(b0) * cin * (4 * m * m), nb * cin, m, at);
+    gather_mode(gs, dout + static_cast<long long>(b0) * cout * (4 * m * m), nb * cout, m, at);
+    __syncthreads();
+    for (int t = threadIdx.x; t < cin * cout; t += blockDim.x) {
+      const int o = t % cout, i = t / cout;
+      float re = b0 ? dwre[wbase + t] : 0.f, im = b0 ? dwim[wbase + t] : 0.f;
+      for (int b = 0; b < nb; ++b) {
+        const float2 yv = ys[b * cin + i], gv = gs[b * cout + o];
+        const float a = yv.x, c = yv.y, gr = gv.x, gi = gv.y;
+        re += __fmaf_rn(a, gr, __fmul_rn(c, gi));
+        im += __fmaf_rn(a, gi, -__fmul_rn(c, gr));
+      }
+      dwre[wbase + t] = re;
+      dwim[wbase + t] = im;
     }
-    dwre[t] = re;
-    dwim[t] = im;
   }
+}
+
+template <bool ADJOINT>
+cudaError_t launch_mode_mix(const float* x, const void* wre, const void* wim, float* out, void* out_bf, int B,
+                            int n_in, int n_out, int m, cudaStream_t stream) {
+  const long long len = ADJOINT ? n_in : n_out;
+  const MixStage st = mix_stage(n_in, static_cast<long long>(n_in) * n_out / len * (len + 2), B);
+  cudaError_t e = cudaFuncSetAttribute(mode_mix_kernel<ADJOINT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(st.bytes));
+  if (e != cudaSuccess) return e;
+  mode_mix_kernel<ADJOINT><<<2 * m * m, 256, st.bytes, stream>>>(
+      x, static_cast<const __nv_bfloat16*>(wre), static_cast<const __nv_bfloat16*>(wim), out,
+      static_cast<__nv_bfloat16*>(out_bf), B, n_in, n_out, m, st);
+  return cudaGetLastError();
 }
 
 // Adam on FP32 master weights; the BF16 copy the GEMMs read is refreshed in the same pass.
@@ -591,7 +680,7 @@ __global__ void mse_kernel(const float* __restrict__ pred, const float* __restri
   }
 }
 
-__device__ int g_gemm_timeouts = 0;  // set when a tcgen05 GEMM's bounded wait gave up
+__device__ int g_gemm_timeouts = 0;  // set when a bounded wait of a tcgen05 kernel gave up
 int g_gemm_engine = 0;                // 0: tcgen05 (default), 1: mma.sync
 
 int grid_for(long long n) {
@@ -600,6 +689,13 @@ int grid_for(long long n) {
 }
 
 }  // namespace
+
+cudaError_t gemm_timeout_flag(int** flag) {
+  return cudaGetSymbolAddress(reinterpret_cast<void**>(flag), g_gemm_timeouts);
+}
+
+int gemm_engine() { return g_gemm_engine; }
+
 }  // namespace pg
 
 extern "C" {
@@ -706,18 +802,48 @@ int pg_fno_gelu_backward(const float* pre, const float* grad_act, float* grad_pr
 int pg_fno_channel_sum(const float* x, float* out, int32_t B, int32_t C, int64_t plane, int32_t accumulate,
                        void* stream) {
   PG_CHECK(x && out && B > 0 && C > 0 && plane > 0, PG_ERR_INVALID, "pg_fno_channel_sum: bad argument");
-  pg::channel_sum_kernel<<<C, 256, 0, static_cast<cudaStream_t>(stream)>>>(x, out, B, C, plane, accumulate);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (plane % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+    constexpr int smem = pg::kSumRing * pg::kSumChunk * 4;
+    PG_CUDA(cudaFuncSetAttribute(pg::channel_sum_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    pg::channel_sum_kernel<true><<<C, 256, smem, st>>>(x, out, B, C, plane, accumulate);
+  } else {
+    pg::channel_sum_kernel<false><<<C, 256, 0, st>>>(x, out, B, C, plane, accumulate);
+  }
   PG_CUDA(cudaGetLastError());
+  return PG_OK;
+}
+
+int pg_fno_mode_mix_bf16(const float* y, const void* wre, const void* wim, float* out, void* out_bf16, int32_t B,
+                         int32_t cin, int32_t cout, int32_t modes, void* stream) {
+  PG_CHECK(y && wre && wim && (out || out_bf16) && B > 0 && cin > 0 && cout > 0 && modes > 0, PG_ERR_INVALID,
+           "pg_fno_mode_mix: bad argument");
+  PG_CUDA(pg::launch_mode_mix<false>(y, wre, wim, out, out_bf16, B, cin, cout, modes,
+                                     static_cast<cudaStream_t>(stream)));
   return PG_OK;
 }
 
 int pg_fno_mode_mix(const float* y, const void* wre, const void* wim, float* out, int32_t B, int32_t cin,
                     int32_t cout, int32_t modes, void* stream) {
-  PG_CHECK(y && wre && wim && out && B > 0 && cin > 0 && cout > 0 && modes > 0, PG_ERR_INVALID,
-           "pg_fno_mode_mix: bad argument");
-  const long long total = static_cast<long long>(B) * cout * 2 * modes * modes;
-  pg::mode_mix_kernel<<<pg::grid_for(total), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      y, static_cast<const __nv_bfloat16*>(wre), static_cast<const __nv_bfloat16*>(wim), out, B, cin, cout, modes);
+  PG_CHECK(out, PG_ERR_INVALID, "pg_fno_mode_mix: bad argument");
+  return pg_fno_mode_mix_bf16(y, wre, wim, out, nullptr, B, cin, cout, modes, stream);
+}
+
+int pg_fno_mode_mix_backward_bf16(const float* y, const float* dout, const void* wre, const void* wim, float* dy,
+                                  void* dy_bf16, float* dwre, float* dwim, int32_t B, int32_t cin, int32_t cout,
+                                  int32_t modes, void* stream) {
+  PG_CHECK(y && dout && wre && wim && B > 0 && cin > 0 && cout > 0 && modes > 0, PG_ERR_INVALID,
+           "pg_fno_mode_mix_backward: bad argument");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dy || dy_bf16)
+    PG_CUDA(pg::launch_mode_mix<true>(dout, wre, wim, dy, dy_bf16, B, cout, cin, modes, st));
+  if (dwre && dwim) {
+    const pg::MixStage m = pg::mix_stage(cin + cout, 1LL << 40, B);
+    PG_CUDA(cudaFuncSetAttribute(pg::mode_mix_back_weight_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(m.bytes)));
+    pg::mode_mix_back_weight_kernel<<<2 * modes * modes, 256, m.bytes, st>>>(y, dout, dwre, dwim, B, cin, cout, modes,
+                                                                             m.samples);
+  }
   PG_CUDA(cudaGetLastError());
   return PG_OK;
 }
@@ -725,22 +851,7 @@ int pg_fno_mode_mix(const float* y, const void* wre, const void* wim, float* out
 int pg_fno_mode_mix_backward(const float* y, const float* dout, const void* wre, const void* wim, float* dy,
                              float* dwre, float* dwim, int32_t B, int32_t cin, int32_t cout, int32_t modes,
                              void* stream) {
-  PG_CHECK(y && dout && wre && wim && B > 0 && cin > 0 && cout > 0 && modes > 0, PG_ERR_INVALID,
-           "pg_fno_mode_mix_backward: bad argument");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (dy) {
-    const long long total = static_cast<long long>(B) * cin * 2 * modes * modes;
-    pg::mode_mix_back_input_kernel<<<pg::grid_for(total), 256, 0, st>>>(
-        dout, static_cast<const __nv_bfloat16*>(wre), static_cast<const __nv_bfloat16*>(wim), dy, B, cin, cout,
-        modes);
-  }
-  if (dwre && dwim) {
-    const long long total = static_cast<long long>(2 * modes) * modes * cin * cout;
-    pg::mode_mix_back_weight_kernel<<<pg::grid_for(total), 256, 0, st>>>(y, dout, dwre, dwim, B, cin, cout,
-                                                                         modes);
-  }
-  PG_CUDA(cudaGetLastError());
-  return PG_OK;
+  return pg_fno_mode_mix_backward_bf16(y, dout, wre, wim, dy, nullptr, dwre, dwim, B, cin, cout, modes, stream);
 }
 
 int pg_fno_adam(float* w, const float* g, float* m1, float* m2, void* w_bf16, int64_t n, float lr,

@@ -1,4 +1,4 @@
-// Inline-PTX helpers for mbarriers and 1-D bulk (TMA) copies, sm_90+ / sm_103a.
+// Inline-PTX helpers for mbarriers and asynchronous copies, sm_90+ / sm_103a.
 #pragma once
 #include <cstdint>
 
@@ -30,6 +30,22 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
           dst),
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
+}
+
+// Per-thread asynchronous copies (both addresses aligned to the size), in commit groups.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // Non-blocking test: has the phase of parity `parity` completed?

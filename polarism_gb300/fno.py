@@ -152,9 +152,106 @@ class FNO2d:
         torch = self.torch
         return torch.empty(shape, dtype=torch.bfloat16 if bf else torch.float32, device=self.device)
 
+    # ------------------------------------------------------------------ fused passes
+    @property
+    def fused(self):
+        """Whether one launch does a layer's pass (``csrc/fno_fused.cu``): the same results as the
+        general GEMMs, which serve every other size and the mma.sync engine."""
+        flag = C.c_int32()
+        self._check(self.lib.pg_fno_fused(self.n, self.modes, max(self.c_in, self.c_out, self.width, self.hidden),
+                                          C.byref(flag)), "pg_fno_fused")
+        return bool(flag.value)
+
+    def _layer(self, wname, v_bf, batch, cin, cout, *, transposed=False, z=None, table=None, rows=False,
+               bias=None, pre=None, mode=0, u=None, out=None):
+        opt = lambda t: _ptr(t) if t is not None else None
+        self._check(self.lib.pg_fno_layer(
+            _ptr(self.w_bf[wname]), 1 if transposed else 0, _ptr(v_bf), opt(z), opt(table), 1 if rows else 0,
+            _ptr(self.w[bias]) if bias is not None else None, opt(pre), opt(u), opt(out), batch, cin, cout,
+            self.n, 2 * self.modes if z is not None else 0, mode, self.stream), "pg_fno_layer")
+
+    def _dft_x(self, v_bf, table, rows, batch):
+        out = self._empty(batch, self.width, self.n, 2 * self.modes, bf=True)
+        self._check(self.lib.pg_fno_dft_x(_ptr(v_bf), _ptr(table), 1 if rows else 0, _ptr(out),
+                                          batch * self.width * self.n, self.n, self.modes, self.stream),
+                    "pg_fno_dft_x")
+        return out
+
+    def _dft_y(self, src_bf, batch, *, inverse):
+        """G src as FP32 (the mode mixing's operand), or G^H src as BF16 (the next GEMM's)."""
+        n, m2 = self.n, 2 * self.modes
+        out = self._empty(batch, self.width, n if inverse else m2, m2, bf=inverse)
+        self._check(self.lib.pg_fno_dft_y(_ptr(self.gre), _ptr(self.gim), _ptr(src_bf),
+                                          None if inverse else _ptr(out), _ptr(out) if inverse else None,
+                                          batch * self.width, n, self.modes, 1 if inverse else 0, self.stream),
+                    "pg_fno_dft_y")
+        return out
+
+    def _forward_fused(self, a):
+        B, n, m, W, H = a.shape[0], self.n, self.modes, self.width, self.hidden
+        cache = {"B": B}
+        cache["a_bf"] = a_bf = self._bf(a.contiguous(), self._empty(B, self.c_in, n, n, bf=True))
+        v_bf = self._empty(B, W, n, n, bf=True)
+        self._layer("lift_w", a_bf, B, self.c_in, W, bias="lift_b", out=v_bf)
+        for l in range(self.layers):
+            cache[f"v{l}_bf"] = v_bf
+            cache[f"Y{l}"] = Y = self._dft_y(self._dft_x(v_bf, self.fx, False, B), B, inverse=False)
+            O_bf = self._empty(B, W, 2 * m, 2 * m, bf=True)
+            self._check(self.lib.pg_fno_mode_mix_bf16(_ptr(Y), _ptr(self.w_bf[f"spec{l}_re"]),
+                                                      _ptr(self.w_bf[f"spec{l}_im"]), None, _ptr(O_bf), B, W, W,
+                                                      m, self.stream), "pg_fno_mode_mix_bf16")
+            Z_bf = self._dft_y(O_bf, B, inverse=True)
+            cache[f"u{l}"] = u = self._empty(B, W, n, n)
+            v_next_bf = self._empty(B, W, n, n, bf=True)
+            self._layer(f"w{l}", v_bf, B, W, W, z=Z_bf, table=self.hx, bias=f"b{l}",
+                        mode=1 if l < self.layers - 1 else 0, u=u, out=v_next_bf)
+            v_bf = v_next_bf
+        cache["vL_bf"] = v_bf
+        cache["h"] = h = self._empty(B, H, n, n)
+        cache["q_bf"] = q_bf = self._empty(B, H, n, n, bf=True)
+        self._layer("proj1_w", v_bf, B, W, H, bias="proj1_b", mode=1, u=h, out=q_bf)
+        out = self._empty(B, self.c_out, n, n)
+        self._layer("proj2_w", q_bf, B, H, self.c_out, bias="proj2_b", u=out)
+        return out, cache
+
+    def _backward_fused(self, cache, dout):
+        B, n, m, W, H = cache["B"], self.n, self.modes, self.width, self.hidden
+        grads = {}
+        dout = dout.contiguous()
+        dout_bf = self._bf(dout, self._empty(*dout.shape, bf=True))
+        self._pointwise_back("proj2_w", cache["q_bf"], dout_bf, dout, B, H, self.c_out, grads, fused=True)
+        dh, dh_bf = self._empty(B, H, n, n), self._empty(B, H, n, n, bf=True)
+        self._layer("proj2_w", dout_bf, B, self.c_out, H, transposed=True, pre=cache["h"], mode=2, u=dh, out=dh_bf)
+        self._pointwise_back("proj1_w", cache["vL_bf"], dh_bf, dh, B, W, H, grads, fused=True)
+        du, du_bf = self._empty(B, W, n, n), self._empty(B, W, n, n, bf=True)
+        self._layer("proj1_w", dh_bf, B, H, W, transposed=True, u=du, out=du_bf)
+        for l in reversed(range(self.layers)):
+            self._pointwise_back(f"w{l}", cache[f"v{l}_bf"], du_bf, du, B, W, W, grads, fused=True)
+            # Spectral adjoint: dZ = du Hx^T, dO = G dZ, (dY, dR) = mixing adjoint, dX = G^H dY,
+            # dv = W^T du + dX Fx^T, times GELU' of the layer below.
+            dO = self._dft_y(self._dft_x(du_bf, self.hx, True, B), B, inverse=False)
+            dY_bf = self._empty(B, W, 2 * m, 2 * m, bf=True)
+            dre = self._empty(2 * m, m, W, W)
+            dim = self._empty(2 * m, m, W, W)
+            self._check(self.lib.pg_fno_mode_mix_backward_bf16(
+                _ptr(cache[f"Y{l}"]), _ptr(dO), _ptr(self.w_bf[f"spec{l}_re"]), _ptr(self.w_bf[f"spec{l}_im"]),
+                None, _ptr(dY_bf), _ptr(dre), _ptr(dim), B, W, W, m, self.stream),
+                "pg_fno_mode_mix_backward_bf16")
+            grads[f"spec{l}_re"], grads[f"spec{l}_im"] = dre, dim
+            dX_bf = self._dft_y(dY_bf, B, inverse=True)
+            dv, dv_bf = self._empty(B, W, n, n), self._empty(B, W, n, n, bf=True)
+            self._layer(f"w{l}", du_bf, B, W, W, transposed=True, z=dX_bf, table=self.fx, rows=True,
+                        pre=cache[f"u{l - 1}"] if l > 0 else None, mode=2 if l > 0 else 0, u=dv, out=dv_bf)
+            du, du_bf = dv, dv_bf
+        self._pointwise_back("lift_w", cache["a_bf"], du_bf, du, B, self.c_in, W, grads, fused=True)
+        return grads
+
     # ------------------------------------------------------------------ forward / backward
     def forward(self, a, keep=True):
         """a: float32 device tensor (B, c_in, n, n).  Returns (out, cache)."""
+        if self.fused:
+            out, cache = self._forward_fused(a)
+            return out, cache if keep else None
         torch = self.torch
         B = a.shape[0]
         n, m, W = self.n, self.modes, self.width
@@ -202,17 +299,22 @@ class FNO2d:
             cache = None
         return out, cache
 
-    def _pointwise_back(self, wname, x_bf, g_bf, g32, batch, cin, cout, grads, dx=None, dx_accumulate=False):
+    def _pointwise_back(self, wname, x_bf, g_bf, g32, batch, cin, cout, grads, dx=None, dx_accumulate=False,
+                        fused=False):
         P = self.n * self.n
         # dW = sum over samples and sites of g x^T: a split-K GEMM (the samples and 4096-site
         # slices of the plane each give one partial product), then a fixed-order sum.
         chunk = 4096 if P % 4096 == 0 else P
         slices = P // chunk
         parts = self._empty(batch * slices, cout, cin)
-        self._check(self.lib.pg_gemm_bf16_2d(
-            _ptr(g_bf), _ptr(x_bf), _ptr(parts), cout, cin, chunk, P, P, cin, 0, 1, 1.0, 0.0,
-            batch, cout * P, cin * P, slices * cout * cin, slices, chunk, chunk, cout * cin,
-            self.stream), "pg_gemm_bf16_2d")
+        if fused:
+            self._check(self.lib.pg_fno_outer(_ptr(g_bf), _ptr(x_bf), _ptr(parts), batch, cout, cin, P, slices,
+                                              self.stream), "pg_fno_outer")
+        else:
+            self._check(self.lib.pg_gemm_bf16_2d(
+                _ptr(g_bf), _ptr(x_bf), _ptr(parts), cout, cin, chunk, P, P, cin, 0, 1, 1.0, 0.0,
+                batch, cout * P, cin * P, slices * cout * cin, slices, chunk, chunk, cout * cin,
+                self.stream), "pg_gemm_bf16_2d")
         dw = self._empty(cout, cin)
         self._check(self.lib.pg_fno_sum_slices(_ptr(parts), _ptr(dw), cout * cin, batch * slices, 0,
                                                self.stream), "pg_fno_sum_slices")
@@ -227,6 +329,8 @@ class FNO2d:
 
     def backward(self, cache, dout):
         """Gradients of sum(dout * out); dout: float32 device tensor like the output."""
+        if self.fused:
+            return self._backward_fused(cache, dout)
         B = cache["B"]
         n, m, W, H = self.n, self.modes, self.width, self.hidden
         grads = {}
