@@ -84,7 +84,7 @@ RK4Route choose_rk4_route(int nx, int ny, int members, int sm_count, const RK4Fe
       // whole turns of the 8-row ring
       const long long blocks = row_blocks(members, ny, static_cast<long long>(sms) * (1024 / nx));
       const double iters = (static_cast<int>(row_iterations(members, ny, blocks)) + 7) / 8 * 8;
-      const double iter = heavy                 ? 1.82
+      const double iter = heavy                 ? 1.78
                           : f.potential == 1    ? 1.64
                           : f.relax             ? 1.41
                           : f.pump_terms == 1   ? 1.13

@@ -734,9 +734,12 @@ int wide_rk4_grid(int nx, int ny, int members, int sm_count, int terms) {
   const long long bands = nx > 1024 ? nx / 1024 : 1;
   const long long rows = static_cast<long long>(members) * bands * ny;
   const long long blocks = static_cast<long long>(per_sm) * std::max(1, sm_count);
-  // Rows that fit a block: all SMs, and no block across two members where that leaves the busiest
-  // one fewer rows (one 1024^2 member: 28 us a step with 64 blocks of 16 rows, 20 with 152).
-  if (nx <= 1024) {
+  // Blocks of 16 rows or more, as many as fit.  Where those leave SMs without a block, or are all that fit, rows
+  // of at most 1024 sites go by whole strips of members instead where that leaves the busiest block
+  // fewer rows (one 1024^2 member: 28 us a step with 64 blocks of 16 rows, 20 with 128 of 8; 64 members of 256^2
+  // with a complex potential 82 and 72; between the two, shorter blocks only add fill: 64 members of 128^2
+  // 19.5 us with 512 blocks of 16 rows, 22 with 1024 of 8).
+  if (nx <= 1024 && (rows / 16 < sm_count || rows / 16 >= blocks)) {
     const long long b = row_blocks(members, ny, blocks);
     if (b % members != 0) return static_cast<int>(b);
     // Iterations come in whole turns of the ring: the fewest strips that need as many turns.
