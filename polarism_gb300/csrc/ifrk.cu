@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(1024) ifrk_col_kernel(typename C2T<T>::type* _
         dsum[q] = acc;
         nval[q] = n0[ridx[q]] + acc;
       }
-      general.apply(v, nval, dsum, ridx, o, local);
+      general.apply(v, nval, dsum, general.load(o), ridx, o, local);
       if (a.mode == 0 || (a.mode == 1 && a.noise)) {
         buf[i * CC + c] = v[0];
         if (comps == 2) buf[i * CC + C + c] = v[1];

@@ -15,8 +15,17 @@
 namespace pg {
 namespace {
 
+// Two components are bound by the latency of the coupled steps, not by registers or warps: a thread
+// takes kPairModes modes through the Lawson terms together (their loads and sines independent of one
+// another) with 128 registers, and the column pass may use twice the registers where more than one
+// block would fit.  A Dormand-Prince trial: 64^2 263 -> 226 us, 256^2 299 -> 260 us, 512^2 432 -> 415 us,
+// 2048^2 4.86 -> 4.66 ms.  Two modes are 2 % slower, one with the next one's loads ahead 6 %; two sites
+// at a time in the column pass spill (512^2 474 us).
+constexpr int kPairModes = 4;
+
 template <int N, int V, int COMPS>
-__global__ void __launch_bounds__(RowShape<N, V, COMPS>::MAX_THREADS, 1024 / RowShape<N, V, COMPS>::MAX_THREADS)
+__global__ void __launch_bounds__(RowShape<N, V, COMPS>::MAX_THREADS,
+                                  (COMPS == 2 ? 512 : 1024) / RowShape<N, V, COMPS>::MAX_THREADS)
     ifrk_row_reg_kernel(const float2* __restrict__ in, float2* __restrict__ save,
                         float2* __restrict__ out, const float2* __restrict__ tables,
                         const float4* __restrict__ tab, const __grid_constant__ IfrkRowArgs a) {
@@ -85,6 +94,7 @@ __global__ void __launch_bounds__(RowShape<N, V, COMPS>::MAX_THREADS, 1024 / Row
         }
       }
     } else {
+      constexpr int U = kPairModes;
       const OwnSlots<N, V> slots(t);
 #pragma unroll
       for (int m = 0; m < V; ++m) buf[slots.slot(m)] = v[m];
@@ -96,26 +106,43 @@ __global__ void __launch_bounds__(RowShape<N, V, COMPS>::MAX_THREADS, 1024 / Row
       const float* modes = a.modes + static_cast<long long>(member) * kSpinModeFields * plane +
                            static_cast<long long>(row) * N + t;
 #pragma unroll 1
-      for (int h = 0; h < V / 2; ++h) {
-        const int m = comp * (V / 2) + h;
-        const SpinMode mode = load_spin_mode(modes + m * M, plane);
-        const int slot = slots.slot(m);
-        const float2 self0 = b0[slot], self1 = b1[slot];
-        const long long at = moff + t + m * M;
-        float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+      for (int h = 0; h < V / 2; h += U) {
+        SpinMode mode[U];
+        float2 self0[U], self1[U], acc0[U], acc1[U];
+        const int m0 = comp * (V / 2) + h;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          mode[u] = load_spin_mode(modes + (m0 + u) * M, plane);
+          const int slot = slots.slot(m0 + u);
+          self0[u] = b0[slot];
+          self1[u] = b1[slot];
+          acc0[u] = acc1[u] = make_float2(0.f, 0.f);
+        }
 #pragma unroll 1
         for (int s = 0; s < a.terms; ++s) {
-          float2 s0 = self0, s1 = self1;
-          if (a.src[s]) {
-            const float2* src = static_cast<const float2*>(a.src[s]) + at;
-            s0 = src[0];
-            s1 = src[plane];
+          float2 s0[U], s1[U];
+          const float2* src = static_cast<const float2*>(a.src[s]);
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            s0[u] = self0[u];
+            s1[u] = self1[u];
+            if (src) {
+              const long long at = moff + t + (m0 + u) * M;
+              s0[u] = src[at];
+              s1[u] = src[at + plane];
+            }
           }
-          spin_term(mode, a.tau_hi[s], a.tau_lo[s], static_cast<float>(a.coef[s] * a.inv_n), zf, inv_hbar,
-                    s0, s1, acc0, acc1);
+          const float w = static_cast<float>(a.coef[s] * a.inv_n);
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            spin_term(mode[u], a.tau_hi[s], a.tau_lo[s], w, zf, inv_hbar, s0[u], s1[u], acc0[u], acc1[u]);
         }
-        b0[slot] = acc0;
-        b1[slot] = acc1;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int slot = slots.slot(m0 + u);
+          b0[slot] = acc0[u];
+          b1[slot] = acc1[u];
+        }
       }
       pair_sync();
 #pragma unroll
@@ -262,7 +289,7 @@ __device__ __forceinline__ void stage_reservoirs(const IfrkColArgs& a, const flo
 // SINGLE: ifrk_sites_batched holds (kernels apart, so that neither path pays the other's registers).
 template <int N, int V, int COMPS, bool SINGLE>
 __global__ void __launch_bounds__(ColShape<float, N, V, COMPS>::MAX_THREADS,
-                                  ColShape<float, N, V, COMPS>::MIN_BLOCKS)
+                                  (ColShape<float, N, V, COMPS>::MIN_BLOCKS + COMPS - 1) / COMPS)
     ifrk_col_reg_kernel(float2* __restrict__ psi, const float* __restrict__ n0,
                         float* __restrict__ dn_out, float* __restrict__ n_out,
                         float2* __restrict__ psi_start, float2* __restrict__ psi_new,
@@ -342,13 +369,14 @@ __global__ void __launch_bounds__(ColShape<float, N, V, COMPS>::MAX_THREADS,
           const int f = Cr == 2 ? (q >> 1) : q, cr = Cr == 2 ? (q & 1) : 0;
           ridx[q] = f * fstride + member * qstride + cr * plane + o;
         }
+        const auto site = general.load(o);
         if (COMPS == 2 && NQ == 4)
           stage_reservoirs<4>(a, n0, ridx, nval, dsum);
         else if (NQ == 2)
           stage_reservoirs<2>(a, n0, ridx, nval, dsum);
         else if (NQ == 1)
           stage_reservoirs<1>(a, n0, ridx, nval, dsum);
-        general.apply(w, nval, dsum, ridx, o, local);
+        general.apply(w, nval, dsum, site, ridx, o, local);
         if (a.mode == 0 || (a.mode == 1 && a.noise)) {
           b0[slot] = w[0];
           if (COMPS == 2) b0[slot + C] = w[1];

@@ -194,7 +194,22 @@ struct IfrkGeneral {
   long long fbase, plane;
   const PhiloxCellPrefix (&prefix)[2];
 
-  __device__ __forceinline__ void apply(C2 (&v)[2], T (&nval)[4], const T (&dsum)[4],
+  // The stage's envelope and potential at site o: loaded with the reservoirs, before any store.
+  struct Site {
+    T pump, vre, vim;
+  };
+  __device__ __forceinline__ Site load(long long o) const {
+    Site p{T(0), T(0), T(0)};
+    if (a.mode != 0) return p;
+    if (a.res_fields >= 1 && !(a.pump_terms > 1 && cs)) p.pump = pm[o];
+    if (vm) {
+      p.vre = a.potential == 2 ? vm[2 * o] : vm[o];
+      p.vim = a.potential == 2 ? vm[2 * o + 1] : T(0);
+    }
+    return p;
+  }
+
+  __device__ __forceinline__ void apply(C2 (&v)[2], T (&nval)[4], const T (&dsum)[4], const Site& site,
                                         const long long (&ridx)[4], long long o, double& local) const {
     const int comps = a.comps, F = a.res_fields, Cr = a.res_comps, NQ = F * Cr;
     const int L = a.pump_terms > 1 ? a.pump_terms : 1;
@@ -206,11 +221,7 @@ struct IfrkGeneral {
         if (comp < comps && psi_start) psi_start[fbase + comp * plane + o] = v[comp];
       }
       C2 out[2];
-      T vre = T(0), vim = T(0);
-      if (vm) {
-        vre = a.potential == 2 ? vm[2 * o] : vm[o];
-        vim = a.potential == 2 ? vm[2 * o + 1] : T(0);
-      }
+      const T vre = site.vre, vim = site.vim;
 #pragma unroll
       for (int comp = 0; comp < 2; ++comp) {
         if (comp >= comps) break;
@@ -231,7 +242,7 @@ struct IfrkGeneral {
         if (comp < comps) v[comp] = out[comp];
       if (F >= 1) {
         const T p_site = L > 1 && cs ? pump_terms_value(pm, a.pump_term_stride, cs, a.members, L, o)
-                                     : mul_rn_i(s0, pm[o]);
+                                     : mul_rn_i(s0, site.pump);
 #pragma unroll
         for (int cr = 0; cr < 2; ++cr) {
           if (cr >= Cr) break;
