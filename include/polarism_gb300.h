@@ -451,6 +451,10 @@ int pg_fno_dft_x(const void* v, const void* table, int32_t table_rows, void* out
 /* Adam on FP32 weights (bias-corrected, optional L2 decay), refreshing the BF16 copy. */
 int pg_fno_adam(float* w, const float* g, float* m1, float* m2, void* w_bf16, int64_t n, float lr,
                 float beta1, float beta2, float eps, int64_t step, float decay, void* stream);
+/* The same for `count` parameters at once: arrays of device pointers (entries of w_bf16 may be NULL). */
+int pg_fno_adam_many(int32_t count, void* const* w, const void* const* g, void* const* m1, void* const* m2,
+                     void* const* w_bf16, const int64_t* n, float lr, float beta1, float beta2, float eps,
+                     int64_t step, float decay, void* stream);
 /* Weighted squared error over C channels of `plane` values: grad = 2 w_c (pred - target) scale;
  * per-block FP64 partial sums of w_c (pred - target)^2 in partials (blocks_used entries). */
 int pg_fno_mse(const float* pred, const float* target, const float* weight, int32_t C, int64_t plane,

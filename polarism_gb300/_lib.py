@@ -148,6 +148,8 @@ SIGNATURES = {
     "pg_fno_outer": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _i64, _i32, _vp]),
     "pg_fno_dft_y": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
     "pg_fno_dft_x": (C.c_int, [_vp, _vp, _i32, _vp, _i64, _i32, _i32, _vp]),
+    "pg_fno_adam_many": (C.c_int, [_i32, _vp, _vp, _vp, _vp, _vp, _vp, C.c_float, C.c_float, C.c_float,
+                                   C.c_float, _i64, C.c_float, _vp]),
     "pg_fno_adam": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _i64, C.c_float, C.c_float, C.c_float,
                               C.c_float, _i64, C.c_float, _vp]),
     "pg_fno_mse": (C.c_int, [_vp, _vp, _vp, _i32, _i64, _vp, _vp, _vp, _i32, _i64, C.c_float,

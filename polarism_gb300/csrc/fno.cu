@@ -637,20 +637,43 @@ cudaError_t launch_mode_mix(const float* x, const void* wre, const void* wim, fl
   return cudaGetLastError();
 }
 
-// Adam on FP32 master weights; the BF16 copy the GEMMs read is refreshed in the same pass.
-__global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m1,
-                            float* __restrict__ m2, __nv_bfloat16* __restrict__ w_bf, long long n,
-                            float lr, float b1, float b2, float eps, float c1, float c2, float decay) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float gi = g[i] + decay * w[i];
-    const float a = b1 * m1[i] + (1.f - b1) * gi;
-    const float b = b2 * m2[i] + (1.f - b2) * gi * gi;
-    m1[i] = a;
-    m2[i] = b;
-    const float v = w[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
-    w[i] = v;
-    if (w_bf) w_bf[i] = __float2bfloat16_rn(v);
+// Adam on FP32 master weights; the BF16 copy the GEMMs read is refreshed in the same pass.  One launch
+// takes up to kAdamTensors parameters, a block 1024 values of one of them: the two dozen parameters of a
+// network, most of a few hundred values, were as many launches of 4 us (91 us a step, and their issue on
+// the host a tenth of a small network's step); together 21 us.
+constexpr int kAdamTensors = 32;
+constexpr int kAdamValues = 1024;
+struct AdamTensor {
+  float* w;
+  const float* g;
+  float* m1;
+  float* m2;
+  __nv_bfloat16* w_bf;
+  long long n;
+};
+struct AdamBatch {
+  AdamTensor t[kAdamTensors];
+  int first[kAdamTensors + 1];  // first block of each
+  int count;
+};
+__global__ void __launch_bounds__(256) adam_kernel(const __grid_constant__ AdamBatch batch, float lr, float b1, float b2,
+                                                   float eps, float c1, float c2, float decay) {
+  int k = 0;
+  while (k + 1 < batch.count && static_cast<int>(blockIdx.x) >= batch.first[k + 1]) ++k;
+  const AdamTensor& t = batch.t[k];
+  const long long base = static_cast<long long>(blockIdx.x - batch.first[k]) * kAdamValues + threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < kAdamValues / 256; ++q) {
+    const long long i = base + q * 256;
+    if (i >= t.n) break;
+    const float gi = __fmaf_rn(decay, t.w[i], t.g[i]);
+    const float a = __fmaf_rn(b1, t.m1[i], __fmul_rn(1.f - b1, gi));
+    const float b = __fmaf_rn(b2, t.m2[i], __fmul_rn(__fmul_rn(1.f - b2, gi), gi));
+    t.m1[i] = a;
+    t.m2[i] = b;
+    const float v = t.w[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
+    t.w[i] = v;
+    if (t.w_bf) t.w_bf[i] = __float2bfloat16_rn(v);
   }
 }
 
@@ -854,16 +877,52 @@ int pg_fno_mode_mix_backward(const float* y, const float* dout, const void* wre,
   return pg_fno_mode_mix_backward_bf16(y, dout, wre, wim, dy, nullptr, dwre, dwim, B, cin, cout, modes, stream);
 }
 
-int pg_fno_adam(float* w, const float* g, float* m1, float* m2, void* w_bf16, int64_t n, float lr,
-                float beta1, float beta2, float eps, int64_t step, float decay, void* stream) {
-  PG_CHECK(w && g && m1 && m2 && n >= 0 && step >= 1, PG_ERR_INVALID, "pg_fno_adam: bad argument");
-  if (n == 0) return PG_OK;
+int pg_fno_adam_many(int32_t count, void* const* w, const void* const* g, void* const* m1, void* const* m2,
+                     void* const* w_bf16, const int64_t* n, float lr, float beta1, float beta2, float eps,
+                     int64_t step, float decay, void* stream) {
+  PG_CHECK(count >= 0 && (count == 0 || (w && g && m1 && m2 && w_bf16 && n)) && step >= 1, PG_ERR_INVALID,
+           "pg_fno_adam: bad argument");
+  for (int k = 0; k < count; ++k)
+    PG_CHECK(w[k] && g[k] && m1[k] && m2[k] && n[k] >= 0, PG_ERR_INVALID, "pg_fno_adam: bad argument");
   const float c1 = 1.f - std::pow(beta1, static_cast<float>(step));
   const float c2 = 1.f - std::pow(beta2, static_cast<float>(step));
-  pg::adam_kernel<<<pg::grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      w, g, m1, m2, static_cast<__nv_bfloat16*>(w_bf16), n, lr, beta1, beta2, eps, c1, c2, decay);
-  PG_CUDA(cudaGetLastError());
+  pg::AdamBatch batch;
+  batch.count = 0;
+  batch.first[0] = 0;
+  auto launch = [&]() -> cudaError_t {
+    if (batch.count == 0) return cudaSuccess;
+    pg::adam_kernel<<<batch.first[batch.count], 256, 0, static_cast<cudaStream_t>(stream)>>>(batch, lr, beta1, beta2,
+                                                                                             eps, c1, c2, decay);
+    batch.count = 0;
+    return cudaGetLastError();
+  };
+  for (int k = 0; k < count; ++k) {
+    // A tensor too long for the block counts of one launch goes in pieces.
+    constexpr long long piece = (1LL << 20) * pg::kAdamValues;
+    for (long long at = 0; at < n[k]; at += piece) {
+      const long long len = n[k] - at < piece ? n[k] - at : piece;
+      if (batch.count == pg::kAdamTensors) PG_CUDA(launch());
+      __nv_bfloat16* bf = static_cast<__nv_bfloat16*>(w_bf16[k]);
+      batch.t[batch.count] = pg::AdamTensor{static_cast<float*>(w[k]) + at, static_cast<const float*>(g[k]) + at,
+                                            static_cast<float*>(m1[k]) + at, static_cast<float*>(m2[k]) + at,
+                                            bf ? bf + at : nullptr, len};
+      batch.first[batch.count + 1] =
+          batch.first[batch.count] + static_cast<int>((len + pg::kAdamValues - 1) / pg::kAdamValues);
+      ++batch.count;
+    }
+  }
+  PG_CUDA(launch());
   return PG_OK;
+}
+
+int pg_fno_adam(float* w, const float* g, float* m1, float* m2, void* w_bf16, int64_t n, float lr,
+                float beta1, float beta2, float eps, int64_t step, float decay, void* stream) {
+  void* const pw[1] = {w};
+  const void* const pg_[1] = {g};
+  void* const p1[1] = {m1};
+  void* const p2[1] = {m2};
+  void* const pb[1] = {w_bf16};
+  return pg_fno_adam_many(1, pw, pg_, p1, p2, pb, &n, lr, beta1, beta2, eps, step, decay, stream);
 }
 
 int pg_fno_mse(const float* pred, const float* target, const float* weight, int32_t C, int64_t plane,

@@ -383,12 +383,13 @@ class FNO2d:
     # ------------------------------------------------------------------ training
     def adam_step(self, grads, lr=1e-3, betas=(0.9, 0.999), eps=1e-8, decay=0.0):
         self.steps += 1
-        for k in self.names:
-            w = self.w[k]
-            self._check(self.lib.pg_fno_adam(_ptr(w), _ptr(grads[k]), _ptr(self.m1[k]), _ptr(self.m2[k]),
-                                             _ptr(self.w_bf[k]), w.numel(), float(lr), float(betas[0]),
-                                             float(betas[1]), float(eps), self.steps, float(decay),
-                                             self.stream), "pg_fno_adam")
+        count = len(self.names)
+        arrays = [(C.c_void_p * count)(*(t[k].data_ptr() for k in self.names))
+                  for t in (self.w, grads, self.m1, self.m2, self.w_bf)]
+        sizes = (C.c_int64 * count)(*(self.w[k].numel() for k in self.names))
+        self._check(self.lib.pg_fno_adam_many(count, *arrays, sizes, float(lr), float(betas[0]), float(betas[1]),
+                                              float(eps), self.steps, float(decay), self.stream),
+                    "pg_fno_adam_many")
 
     def mse(self, out, target, channel_weight=None, want_grad=True):
         """(loss, grad): mean over all values of w_c (out - target)^2 (FP64 reduction)."""

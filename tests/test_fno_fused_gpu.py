@@ -74,3 +74,45 @@ def test_channel_sum_keeps_the_order_of_its_sum(cuda_lib, B, C, plane):
     for o in (16, 8, 4, 2, 1):
         p[:, :o] = p[:, :o] + p[:, o:2 * o]
     assert np.array_equal(out.cpu().numpy(), p[:, 0])
+
+
+def test_adam_takes_many_parameters_in_one_launch(cuda_lib):
+    """More parameters than one launch takes, empty ones and lengths around a block's 1024 values,
+    against the formula in FP64 (FP32 rounding of a few operations: 1e-6) and each one by itself."""
+    import ctypes
+
+    import torch
+
+    from polarism_gb300 import _lib
+
+    lib = _lib.load()
+    sizes = [1, 1023, 1024, 1025, 0, 5000] + [7 + k for k in range(40)]
+    rng = np.random.default_rng(0)
+    host = [[rng.standard_normal(n).astype(np.float32) for _ in range(3)] +
+            [rng.random(n).astype(np.float32)] for n in sizes]
+    args = (1e-3, 0.9, 0.999, 1e-8, 3, 0.01)
+
+    def run(many):
+        dev = [[torch.tensor(a, device="cuda") for a in t] for t in host]
+        bf = [torch.empty(max(n, 1), dtype=torch.bfloat16, device="cuda") for n in sizes]
+        keep = [torch.empty(1, device="cuda")]
+        ptr = lambda t: t.data_ptr() or keep[0].data_ptr()
+        if many:
+            cols = [(ctypes.c_void_p * len(sizes))(*(ptr(d[c]) for d in dev)) for c in (0, 1, 2, 3)]
+            cols.append((ctypes.c_void_p * len(sizes))(*(b.data_ptr() for b in bf)))
+            _lib.check(lib.pg_fno_adam_many(len(sizes), *cols, (ctypes.c_int64 * len(sizes))(*sizes), *args, None),
+                       "pg_fno_adam_many")
+        else:
+            for d, b, n in zip(dev, bf, sizes):
+                _lib.check(lib.pg_fno_adam(*(ptr(t) for t in d), b.data_ptr(), n, *args, None), "pg_fno_adam")
+        return [[t.cpu().numpy() for t in d] for d in dev], [b[:n].float().cpu().numpy() for b, n in zip(bf, sizes)]
+
+    got, got_bf = run(True)
+    one, one_bf = run(False)
+    for k, (w, g, m1, m2) in enumerate(host):
+        assert all(np.array_equal(x, y) for x, y in zip(got[k], one[k])) and np.array_equal(got_bf[k], one_bf[k])
+        w, g, m1, m2 = (x.astype(np.float64) for x in (w, g, m1, m2))
+        gi = g + 0.01 * w
+        a, b = 0.9 * m1 + 0.1 * gi, 0.999 * m2 + 0.001 * gi * gi
+        v = w - 1e-3 * (a / (1 - 0.9 ** 3)) / (np.sqrt(b / (1 - 0.999 ** 3)) + 1e-8)
+        np.testing.assert_allclose(got[k][0], v, rtol=1e-6, atol=1e-6)
