@@ -1,6 +1,6 @@
 // The site step of the IFRK column passes for the common configuration (device code shared by
 // the generic column pass in ifrk.cu and the 1024-point register-resident column pass in
-// split_fast.cu): one field component, one single reservoir, one laser.  Math as
+// ifrk_col_fast.cu): one field component, one single reservoir, one laser.  Math as
 // polarism/solver/ifrk_fft_cuda_solver.py:128-142 (right-hand side) and :148-241 (stage
 // reservoir n0 + sum_j coef_j dn_j, single-reservoir derivative, step-end clamp and Wigner
 // increment), restated from the generic loop of ifrk_col_kernel, which covers every other

@@ -1,5 +1,5 @@
 // The split-step's local operations at one site (device code shared by the generic column
-// pass in split.cu and the 1024-point register-resident column pass in split_fast.cu): the
+// pass in split.cu and the register-resident column pass in split_reg.cu): the
 // reservoir half steps, the exact nonlinear step and the Wigner increment, for every
 // SplitOp.
 #pragma once
