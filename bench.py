@@ -339,11 +339,6 @@ def run_ours(args):
                     pump_per_member=True, potential=pot_kind)
     if args.rk4_kernel != "auto":
         eng.set_kernel({"wide": 2, "tiled": 1, "wide4": 3}[args.rk4_kernel])
-    kernel_name = ("tiled" if eng.kernel() == 1 else
-                   "full-width, four sites a thread" if eng.kernel() == 3 else
-                   "full-width" if NX <= 1024 else
-                   f"full-width, clusters of {NX // 1024} CTAs (1024-site bands)" if NX <= 8192 else
-                   "full-width, 1024-site bands with recomputed halo")
     eng.set_pump(w["env"])
     if args.potential != "none":
         # A harmonic trap (real part) and an absorbing rim (imaginary part), shared by members.
@@ -358,6 +353,11 @@ def run_ours(args):
             eng.set_potential(trap.astype(np.float32))
     eng.set_noise(w["seeds"], PHYSICS["gamma_C"], PHYSICS["R"], 1.0, DT / (4 * w["dx"] * w["dy"]))
     eng.set_state(w["psi"], w["n"])
+    kernel_name = {1: "tiled", 3: "full-width, four sites a thread", 4: "two-dimensional tiles",
+                   5: "windows of rows"}.get(eng.kernel()) or (
+                   "full-width" if NX <= 1024 else
+                   f"full-width, clusters of {NX // 1024} CTAs (1024-site bands)" if NX <= 8192 else
+                   "full-width, 1024-site bands with recomputed halo")
     stream = torch.cuda.ExternalStream(eng.stream)
     total = args.warmup + args.steps
     scales = np.full((total, 3, members), P0)

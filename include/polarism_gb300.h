@@ -255,8 +255,8 @@ int pg_field_norms_noalloc(const void* psi, int32_t precision, int32_t members,
  * rows of at most 1024 sites; real or complex potential and kinetic relaxation in its general
  * variant), 3 the full-width kernel
  * with four sites a thread (rows of 512 or 1024 sites, no potential or relaxation; bitwise the
- * same results as 2).  pg_rk4_get_kernel reports the kind a grid is eligible for (1, 2 or 3): 2 or
- * 3 also where the automatic choice runs tiles or windows in its place. */
+ * same results as 2).  pg_rk4_get_kernel reports the kernel in use: 1, 2 or 3 as above, 4 the
+ * two-dimensional tiles, 5 the windows of rows (4 and 5 are the automatic choice's alone). */
 int pg_rk4_set_kernel(pg_solver* s, int32_t kind);
 int pg_rk4_get_kernel(pg_solver* s, int32_t* kind);
 

@@ -204,26 +204,32 @@ pg::RK4Route route(const pg_solver* s) {
   return s->route;
 }
 
+pg::WideGeom wide_geometry(const pg_solver* s) {
+  const pg::RK4Features f = features(s);
+  pg::WideGeom w{};
+  w.nx = s->cfg.nx;
+  w.ny = s->cfg.ny;
+  w.members = s->cfg.members;
+  w.blocks = s->wide_blocks;
+  w.pump_stride = s->cfg.pump_per_member ? s->plane : 0;
+  w.pump_terms = f.pump_terms;
+  w.pump_term_stride = s->pump_term_stride;
+  w.halt = s->halt;
+  w.pot = static_cast<const float*>(s->potential);
+  w.pot_stride = s->cfg.potential_per_member ? s->plane : 0;
+  w.pot_kind = f.potential;
+  w.relax = f.relax;
+  w.wait_limit = s->wait_limit;
+  return w;
+}
+
 // Launch one RK4 step reading buffers of parity `from`; step_offset indexes the chunk scales.
 cudaError_t launch_step(pg_solver* s, int from, int step_offset) {
   const int to = 1 - from;
   const pg::RK4Features f = features(s);
   const pg::RK4Route kind = route(s);
   if (kind == pg::RK4Route::kWide) {
-    pg::WideGeom w{};
-    w.nx = s->cfg.nx;
-    w.ny = s->cfg.ny;
-    w.members = s->cfg.members;
-    w.blocks = s->wide_blocks;
-    w.pump_stride = s->cfg.pump_per_member ? s->plane : 0;
-    w.pump_terms = f.pump_terms;
-    w.pump_term_stride = s->pump_term_stride;
-    w.halt = s->halt;
-    w.pot = static_cast<const float*>(s->potential);
-    w.pot_stride = s->cfg.potential_per_member ? s->plane : 0;
-    w.pot_kind = f.potential;
-    w.relax = f.relax;
-    w.wait_limit = s->wait_limit;
+    pg::WideGeom w = wide_geometry(s);
     if (use_quad(s, w)) {
       w.blocks = s->quad_blocks;
       return pg::launch_rk4_quad(static_cast<const float*>(s->psi[from]),
@@ -617,7 +623,12 @@ int pg_rk4_prepare(pg_solver* s, int32_t n_steps) {
 
 int pg_rk4_get_kernel(pg_solver* s, int32_t* kind) {
   PG_CHECK(s && kind, PG_ERR_INVALID, "pg_rk4_get_kernel: null argument");
-  *kind = !use_wide(s) ? 1 : s->rk4_kernel == 3 ? 3 : 2;
+  switch (route(s)) {
+    case pg::RK4Route::kStream: *kind = 1; break;
+    case pg::RK4Route::kWide: *kind = use_quad(s, wide_geometry(s)) ? 3 : 2; break;
+    case pg::RK4Route::kTile: *kind = 4; break;
+    case pg::RK4Route::kWindow: *kind = 5; break;
+  }
   return PG_OK;
 }
 

@@ -250,6 +250,8 @@ class RK4Engine:
         _lib.check(self.lib.pg_set_wait_limit(self.handle, int(polls)), "pg_set_wait_limit")
 
     def kernel(self) -> int:
+        """The RK4 kernel in use: 1, 2 or 3 as in ``set_kernel``, 4 two-dimensional tiles,
+        5 windows of rows."""
         k = C.c_int32()
         _lib.check(self.lib.pg_rk4_get_kernel(self.handle, C.byref(k)), "pg_rk4_get_kernel")
         return k.value
