@@ -259,6 +259,11 @@ int pg_field_norms_noalloc(const void* psi, int32_t precision, int32_t members,
  * two-dimensional tiles, 5 the windows of rows (4 and 5 are the automatic choice's alone). */
 int pg_rk4_set_kernel(pg_solver* s, int32_t kind);
 int pg_rk4_get_kernel(pg_solver* s, int32_t* kind);
+/* The automatic choice for a configuration on a GPU of `sm_count` SMs (0: 152), without one: plan[0] the
+ * kernel as pg_rk4_get_kernel reports it; then the streaming kernel's tile width and strip height, or
+ * the tile shape's index, or the window's capacity in columns, its bands a row and its blocks.  `relax`: a
+ * member has a kinetic relaxation term. */
+int pg_rk4_plan(const pg_config* cfg, int32_t relax, int32_t sm_count, int32_t plan[4]);
 
 /* Failure detection of the TMA-fed RK4 kernels (full-width, four-sites-a-thread, cluster
  * form; no counterpart in the reference, whose kernels wait on nothing).  Every wait of these

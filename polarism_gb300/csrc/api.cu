@@ -201,7 +201,7 @@ bool use_quad(const pg_solver* s, const pg::WideGeom& w) {
 pg::RK4Route route(const pg_solver* s) {
   if (s->rk4_kernel == 1 || (s->rk4_kernel == 0 && s->geom_set && !use_wide(s))) return pg::RK4Route::kStream;
   if (s->rk4_kernel >= 2) return pg::RK4Route::kWide;
-  return s->route;
+  return s->plan.route;
 }
 
 pg::WideGeom wide_geometry(const pg_solver* s) {
@@ -249,7 +249,7 @@ cudaError_t launch_step(pg_solver* s, int from, int step_offset) {
                                static_cast<float>(s->cfg.dt), s->noise, w, s->err_flag, s->stream);
   }
   if (kind == pg::RK4Route::kWindow) {
-    pg::WindowGeom w = s->window;
+    pg::WindowGeom w = s->plan.window;
     w.pump_stride = s->cfg.pump_per_member ? s->plane : 0;
     w.pump_terms = f.pump_terms;
     w.pump_term_stride = s->pump_term_stride;
@@ -273,13 +273,13 @@ cudaError_t launch_step(pg_solver* s, int from, int step_offset) {
   if (kind == pg::RK4Route::kTile) {
     if (s->cfg.precision == PG_DOUBLE)
       return pg::launch_rk4_tile_f64(
-          s->tile_shape, static_cast<const double*>(s->psi[from]), static_cast<const double*>(s->res[from]),
+          s->plan.tile, static_cast<const double*>(s->psi[from]), static_cast<const double*>(s->res[from]),
           static_cast<const double*>(s->pump), static_cast<const double*>(s->potential),
           static_cast<double*>(s->psi[to]), static_cast<double*>(s->res[to]),
           static_cast<const pg::RhsConst<double>*>(s->consts), static_cast<const double*>(s->scales),
           s->step_base, step_offset, s->cfg.dt, s->noise, g, f, s->stream);
     return pg::launch_rk4_tile_f32(
-        s->tile_shape, static_cast<const float*>(s->psi[from]), static_cast<const float*>(s->res[from]),
+        s->plan.tile, static_cast<const float*>(s->psi[from]), static_cast<const float*>(s->res[from]),
         static_cast<const float*>(s->pump), static_cast<const float*>(s->potential),
         static_cast<float*>(s->psi[to]), static_cast<float*>(s->res[to]),
         static_cast<const pg::RhsConst<float>*>(s->consts), static_cast<const float*>(s->scales),
@@ -471,17 +471,8 @@ int pg_create(const pg_config* cfg, const pg_physics* physics, pg_solver** out) 
     if ((e = cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming)) != cudaSuccess)
       return fail(e, "staging event");
   }
-  pg::choose_rk4_geometry(cfg->nx, cfg->ny, cfg->members, cfg->precision, s->sm_count, &s->geom);
-  if (cfg->precision == PG_DOUBLE) {
-    // The tile kernel steps every FP64 grid: measured without / with Wigner noise, us a step,
-    // streaming kernel -> tile kernel: 92.6 -> 11.4 / 141 -> 14.7 at 128^2, 179 -> 24.4 / 269 ->
-    // 35.9 at 256^2, 208 -> 78 / 314 -> 123 at 512^2, 310 -> 268 / 495 -> 426 at 1024^2.
-    s->route = pg::RK4Route::kTile;
-    s->tile_shape = pg::choose_rk4_tile_f64(cfg->nx, cfg->ny, cfg->members, s->sm_count);
-  } else {
-    s->route = pg::choose_rk4_route(cfg->nx, cfg->ny, cfg->members, s->sm_count, features(s), s->geom,
-                                    &s->window, &s->tile_shape);
-  }
+  s->plan = pg::plan_rk4(*cfg, features(s), s->sm_count);
+  s->geom = s->plan.stream;
   int rc = upload_consts(s);
   if (rc != PG_OK) {
     release(s);
@@ -617,6 +608,37 @@ int pg_rk4_prepare(pg_solver* s, int32_t n_steps) {
       }
     }
     done += len;
+  }
+  return PG_OK;
+}
+
+int pg_rk4_plan(const pg_config* cfg, int32_t relax, int32_t sm_count, int32_t plan[4]) {
+  PG_CHECK(cfg && plan && cfg->nx >= 4 && cfg->ny >= 4 && cfg->members >= 1, PG_ERR_INVALID,
+           "pg_rk4_plan: bad argument");
+  pg::RK4Features f{};
+  f.potential = cfg->potential;
+  f.reservoir = cfg->reservoir;
+  f.pump_terms = std::max(1, cfg->pump_terms);
+  f.relax = relax ? 1 : 0;
+  const pg::RK4Plan p = pg::plan_rk4(*cfg, f, sm_count);
+  plan[1] = plan[2] = plan[3] = 0;
+  switch (p.route) {
+    case pg::RK4Route::kStream:
+      plan[0] = 1;
+      plan[1] = p.stream.tile_w;
+      plan[2] = p.stream.strip_h;
+      break;
+    case pg::RK4Route::kWide: plan[0] = 2; break;
+    case pg::RK4Route::kTile:
+      plan[0] = 4;
+      plan[1] = p.tile;
+      break;
+    case pg::RK4Route::kWindow:
+      plan[0] = 5;
+      plan[1] = p.window.wmax;
+      plan[2] = p.window.bands;
+      plan[3] = p.window.blocks;
+      break;
   }
   return PG_OK;
 }

@@ -95,6 +95,8 @@ cudaError_t launch_rk4_step(const T* psi_in, const T* n_in, const T* pump, const
                             int step_offset, T dt, bool noise, const RK4Geom& g,
                             const RK4Features& f, cudaStream_t stream);
 
+constexpr long long kMaxGridYZ = 65535;  // blocks along y or z of a launch
+
 // The same step on two-dimensional tiles (rk4_tile.cuh), bit for bit; `shape` indexes the tile
 // shapes, choose_rk4_tile_f64 picks one for a grid.
 int choose_rk4_tile_f64(int nx, int ny, int members, int sm_count);
@@ -120,11 +122,6 @@ void choose_rk4_geometry(int nx, int ny, int members, int precision, int sm_coun
 int philox_words_device(const uint32_t* counters, uint64_t key, uint32_t* out, int64_t n,
                         cudaStream_t stream);
 
-struct WindowGeom;
-// The kernel an FP32 grid is stepped with when the caller leaves the choice (rk4_plan.cu); fills the
-// window's geometry or the tile's shape for it.
 enum class RK4Route { kStream, kWide, kWindow, kTile };
-RK4Route choose_rk4_route(int nx, int ny, int members, int sm_count, const RK4Features& f,
-                          const RK4Geom& stream, WindowGeom* window, int* tile);
 
 }  // namespace pg

@@ -1,4 +1,7 @@
-// Which kernel steps an FP32 grid when the caller leaves the choice: the tile kernel (rk4_tile.cuh),
+// Which kernel steps a grid when the caller leaves the choice.  FP64: the tile kernel (rk4_tile_f64.cu;
+// measured without / with Wigner noise, us a step, streaming kernel -> tile kernel: 92.6 -> 11.4 /
+// 141 -> 14.7 at 128^2, 179 -> 24.4 / 269 -> 35.9 at 256^2, 208 -> 78 / 314 -> 123 at 512^2,
+// 310 -> 268 / 495 -> 426 at 1024^2), where its launch fits.  FP32: the tile kernel (rk4_tile.cuh),
 // the window kernel (rk4_window.cuh), the full-width kernel (rk4_wide.cu) or the streaming kernel
 // (rk4.cu).  All give the same bits, so the choice is the smallest modelled time.
 //
@@ -41,21 +44,26 @@ double stream_time(const RK4Geom& g, bool general, bool two, int lasers, int sms
   return 2.5 + waves * iters * t;
 }
 
-// Time of the tile shapes of rk4_tile_f32.cu, {width, height, base, slope} without and with the
-// general right-hand side.
+// The tile shapes of rk4_tile_f32.cu.
+constexpr int kTileW[4] = {16, 16, 32, 32}, kTileH[4] = {8, 16, 16, 32};
+
+long long tile_rows(int shape, int ny) { return (ny + static_cast<long long>(kTileH[shape]) - 1) / kTileH[shape]; }
+
+// Their times, {base, slope} without and with the general right-hand side.
 double tile_time(int shape, int nx, int ny, int members, bool general, int sms) {
-  static const double fit[4][6] = {{16, 8, 3.4, 0.92, 3.4, 1.95},
-                                   {16, 16, 4.2, 1.05, 3.9, 2.75},
-                                   {32, 16, 4.0, 1.65, 4.0, 4.2},
-                                   {32, 32, 3.3, 3.45, 2.2, 7.5}};
+  static const double fit[4][4] = {{3.4, 0.92, 3.4, 1.95},
+                                   {4.2, 1.05, 3.9, 2.75},
+                                   {4.0, 1.65, 4.0, 4.2},
+                                   {3.3, 3.45, 2.2, 7.5}};
   const double* f = fit[shape];
-  const long long tiles = static_cast<long long>((nx + f[0] - 1) / f[0]) *
-                          static_cast<long long>((ny + f[1] - 1) / f[1]) * members;
+  const long long tiles = (nx + static_cast<long long>(kTileW[shape]) - 1) / kTileW[shape] * tile_rows(shape, ny) * members;
   const double w = static_cast<double>((tiles + sms - 1) / sms);
-  return general ? f[4] + f[5] * w : f[2] + f[3] * w;
+  return general ? f[2] + f[3] * w : f[0] + f[1] * w;
 }
 
 }  // namespace
+
+namespace {
 
 RK4Route choose_rk4_route(int nx, int ny, int members, int sm_count, const RK4Features& f,
                           const RK4Geom& stream, WindowGeom* window, int* tile) {
@@ -63,8 +71,13 @@ RK4Route choose_rk4_route(int nx, int ny, int members, int sm_count, const RK4Fe
   const bool two = f.reservoir >= 2;
   const bool general = f.potential != 0 || f.relax != 0 || f.reservoir != 1 || f.pump_terms > 1;
   RK4Route route = RK4Route::kStream;
+  // The streaming and tile kernels launch a block a member and strip, the others any number of rows
+  // on a persistent grid.
+  const bool members_fit = members <= kMaxGridYZ;
   double best = 1.12 * stream_time(stream, general, two, f.pump_terms, sms);
-  for (int s = 0; s < 4; ++s) {
+  if (!members_fit || (ny + stream.strip_h - 1) / stream.strip_h > kMaxGridYZ) best = 1e300;
+  for (int s = 0; s < 4 && members_fit; ++s) {
+    if (tile_rows(s, ny) > kMaxGridYZ) continue;
     const double t = tile_time(s, nx, ny, members, general, sms) * (1.0 + 0.2 * (f.pump_terms - 1));
     if (t < best) {
       best = t;
@@ -74,6 +87,7 @@ RK4Route choose_rk4_route(int nx, int ny, int members, int sm_count, const RK4Fe
   }
   if (f.reservoir == 1 && f.pump_terms <= 2) {
     double t = choose_rk4_window(nx, ny, members, sms, window);
+    if (t < 0.0) t = 1e300;  // no window fits
     const bool heavy = f.potential == 2;
     t = 2.5 + t * (heavy ? 1.7 : f.pump_terms == 2 ? 1.3 : f.potential ? 1.12 : f.relax ? 1.1 : 1.0);
     if (t < best) {
@@ -95,6 +109,20 @@ RK4Route choose_rk4_route(int nx, int ny, int members, int sm_count, const RK4Fe
     }
   }
   return route;
+}
+
+}  // namespace
+
+RK4Plan plan_rk4(const pg_config& c, const RK4Features& f, int sm_count) {
+  RK4Plan p;
+  choose_rk4_geometry(c.nx, c.ny, c.members, c.precision, sm_count, &p.stream);
+  if (c.precision == PG_DOUBLE) {
+    p.tile = choose_rk4_tile_f64(c.nx, c.ny, c.members, sm_count);
+    p.route = p.tile >= 0 ? RK4Route::kTile : RK4Route::kStream;
+  } else {
+    p.route = choose_rk4_route(c.nx, c.ny, c.members, sm_count, f, p.stream, &p.window, &p.tile);
+  }
+  return p;
 }
 
 }  // namespace pg

@@ -14,7 +14,8 @@ namespace pg {
 // units of a tile.  Small tiles spread a small grid over the SMs, large ones recompute less: us a
 // step for 16 x 8 / 16 x 16 / 32 x 16 / 32 x 32 tiles (no noise) 11.4 / 16.0 / 24.2 / 40.2 at
 // 128^2, 33.1 / 27.0 / 24.4 / 40.5 at 256^2, 106 / 82 / 81 / 78 at 512^2, 396 / 303 / 272 / 268 at
-// 1024^2; the rule takes the fastest in each.
+// 1024^2; the rule takes the fastest in each.  -1: no launch holds the grid (its y and z dimensions count
+// tile rows and members).
 int choose_rk4_tile_f64(int nx, int ny, int members, int sm_count) {
   const long long sms = sm_count > 0 ? sm_count : 152;
   struct Shape { int w, h, units; };
@@ -22,9 +23,11 @@ int choose_rk4_tile_f64(int nx, int ny, int members, int sm_count) {
                           {16, 16, TileShape<16, 16>::units()},
                           {32, 16, TileShape<32, 16>::units()},
                           {32, 32, TileShape<32, 32>::units()}};
-  int best = 0;
+  int best = -1;
   long long best_cost = -1;
+  if (members > kMaxGridYZ) return best;
   for (int i = 0; i < 4; ++i) {
+    if ((ny + static_cast<long long>(shapes[i].h) - 1) / shapes[i].h > kMaxGridYZ) continue;
     const long long tiles = static_cast<long long>((nx + shapes[i].w - 1) / shapes[i].w) *
                             ((ny + shapes[i].h - 1) / shapes[i].h) * members;
     const long long cost = (tiles + sms - 1) / sms * shapes[i].units;

@@ -43,9 +43,7 @@ struct pg_solver {
   double dt_over_4dv = 0.0;
   pg::RK4Geom geom{};
   bool geom_set = false;     // pg_rk4_set_geometry chose it: the streaming kernel runs with it
-  pg::WindowGeom window{};   // FP32: geometry of the window kernel
-  int tile_shape = 0;        // tile of the tile kernel (choose_rk4_tile_f64, choose_rk4_route)
-  pg::RK4Route route = pg::RK4Route::kStream;  // FP32: the automatic choice
+  pg::RK4Plan plan;          // the automatic choice of RK4 kernel
   // Pinned staging ring for chunk scales and the step base.
   struct Slot {
     void* host = nullptr;

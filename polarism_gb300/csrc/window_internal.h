@@ -22,9 +22,20 @@ struct WindowGeom {
   int relax;
 };
 
+// The kernel a grid is stepped with when the caller leaves the choice, and the geometry of each
+// (rk4_plan.cu).
+struct RK4Plan {
+  RK4Route route = RK4Route::kStream;
+  RK4Geom stream{};
+  WindowGeom window{};  // FP32
+  int tile = 0;         // tile shape of rk4_tile_f32.cu / rk4_tile_f64.cu
+};
+RK4Plan plan_rk4(const pg_config& cfg, const RK4Features& f, int sm_count);
+
 double row_iterations(long long units, int ny, long long blocks);
 long long row_blocks(long long units, int ny, long long slots);
-// Picks bands, band_w, wmax and blocks for a grid; the modelled time in us.
+// Picks bands, band_w, wmax and blocks for a grid; the modelled time in us, negative if no window holds
+// it (rows beyond some 500,000 sites).
 double choose_rk4_window(int nx, int ny, int members, int sm_count, WindowGeom* g);
 cudaError_t launch_rk4_window(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
                               float* n_out, const RhsConst<float>* consts, const float* scales,
