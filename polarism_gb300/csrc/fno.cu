@@ -628,8 +628,7 @@ cudaError_t launch_mode_mix(const float* x, const void* wre, const void* wim, fl
                             int n_in, int n_out, int m, cudaStream_t stream) {
   const long long len = ADJOINT ? n_in : n_out;
   const MixStage st = mix_stage(n_in, static_cast<long long>(n_in) * n_out / len * (len + 2), B);
-  cudaError_t e = cudaFuncSetAttribute(mode_mix_kernel<ADJOINT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(st.bytes));
+  const cudaError_t e = allow_smem(mode_mix_kernel<ADJOINT>);
   if (e != cudaSuccess) return e;
   mode_mix_kernel<ADJOINT><<<2 * m * m, 256, st.bytes, stream>>>(
       x, static_cast<const __nv_bfloat16*>(wre), static_cast<const __nv_bfloat16*>(wim), out,
@@ -862,8 +861,7 @@ int pg_fno_mode_mix_backward_bf16(const float* y, const float* dout, const void*
     PG_CUDA(pg::launch_mode_mix<true>(dout, wre, wim, dy, dy_bf16, B, cout, cin, modes, st));
   if (dwre && dwim) {
     const pg::MixStage m = pg::mix_stage(cin + cout, 1LL << 40, B);
-    PG_CUDA(cudaFuncSetAttribute(pg::mode_mix_back_weight_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(m.bytes)));
+    PG_CUDA(pg::allow_smem(pg::mode_mix_back_weight_kernel));
     pg::mode_mix_back_weight_kernel<<<2 * modes * modes, 256, m.bytes, st>>>(y, dout, dwre, dwim, B, cin, cout, modes,
                                                                              m.samples);
   }

@@ -25,7 +25,6 @@ namespace {
 using bf16 = __nv_bfloat16;
 
 constexpr int kThreads = 128;
-constexpr int kMaxSmem = 227 * 1024;
 // Layouts: the strides between core matrices carry 16 spare bytes where neighbouring lanes of a copy
 // would otherwise write the same banks.
 constexpr int kMnChunk = 144;              // M-major operand of 128 rows: 8 rows of M to the next 8
@@ -558,11 +557,6 @@ int sm_count() {
   return sms;
 }
 
-template <typename K>
-cudaError_t set_smem(K kernel, int bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
 template <bool INVERSE>
 int run_dft_y(const pg::DftYArgs& in, int batch, cudaStream_t stream) {
   DftYArgs a = in;
@@ -570,7 +564,7 @@ int run_dft_y(const pg::DftYArgs& in, int batch, cudaStream_t stream) {
   PG_CHECK(smem <= kMaxSmem, PG_ERR_UNSUPPORTED, "pg_fno_dft_y: does not fit shared memory");
   int* flag = nullptr;
   PG_CUDA(gemm_timeout_flag(&flag));
-  PG_CUDA(set_smem(dft_y_kernel<INVERSE>, smem));
+  PG_CUDA(allow_smem(dft_y_kernel<INVERSE>));
   dft_y_kernel<INVERSE><<<dim3(batch, (a.M + 127) / 128), kThreads, smem, stream>>>(a, flag);
   PG_CUDA(cudaGetLastError());
   return PG_OK;
@@ -637,7 +631,7 @@ int pg_fno_layer(const void* w, int32_t w_transposed, const void* v, const void*
   int* flag = nullptr;
   PG_CUDA(pg::gemm_timeout_flag(&flag));
   auto kernel = mode == 2 ? pg::layer_kernel<2> : mode == 1 ? pg::layer_kernel<1> : pg::layer_kernel<0>;
-  PG_CUDA(pg::set_smem(kernel, smem));
+  PG_CUDA(pg::allow_smem(kernel));
   const int per_sm = std::min({pg::kLayerBlocks, 512 / a.cols, 228 * 1024 / (smem + 1024)});
   const int tiles = (n + 127) / 128;
   const int resident = std::max(1, per_sm * pg::sm_count() / tiles);
@@ -673,7 +667,7 @@ int pg_fno_outer(const void* g, const void* x, float* parts, int32_t B, int32_t 
   const int blocks = B * slices;
   auto run = [&](auto kernel, int slabs) {
     const int smem = pg::block_smem(slabs * stage + 2048, a.cols);
-    const cudaError_t e = pg::set_smem(kernel, smem);
+    const cudaError_t e = pg::allow_smem(kernel, 1024);
     if (e != cudaSuccess) return e;
     kernel<<<blocks, pg::kOuterThreads, smem, st>>>(a, flag);
     return cudaGetLastError();
@@ -730,7 +724,7 @@ int pg_fno_dft_x(const void* v, const void* table, int32_t table_rows, void* out
   PG_CHECK(smem <= pg::kMaxSmem, PG_ERR_UNSUPPORTED, "pg_fno_dft_x: does not fit shared memory");
   int* flag = nullptr;
   PG_CUDA(pg::gemm_timeout_flag(&flag));
-  PG_CUDA(pg::set_smem(pg::dft_x_kernel, smem));
+  PG_CUDA(pg::allow_smem(pg::dft_x_kernel));
   pg::dft_x_kernel<<<static_cast<unsigned>((rows + 127) / 128), pg::kThreads, smem,
                      static_cast<cudaStream_t>(stream)>>>(a, flag);
   PG_CUDA(cudaGetLastError());

@@ -9,6 +9,17 @@ cudaError_t gemm_timeout_flag(int** flag);
 // 0: tcgen05, 1: mma.sync (pg_gemm_set_engine).
 int gemm_engine();
 
+// Shared memory of a block at most.
+constexpr int kMaxSmem = 227 * 1024;
+
+// Allows `kernel` all of it but `fixed` bytes of static shared memory.  The limit belongs to the
+// kernel on a device, not to a launch: every caller asks for the same one, whatever its launch takes,
+// so that one thread's small launch never lowers the limit under another's large one.
+template <typename K>
+cudaError_t allow_smem(K* kernel, int fixed = 0) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem - fixed);
+}
+
 // GELU in its tanh form and its derivative.
 constexpr float kGeluC = 0.7978845608028654f;  // sqrt(2 / pi)
 
