@@ -570,12 +570,13 @@ long long count_items(const pg_sweep* w, int lanes, int rows) {
   return items;
 }
 
-// The shortest strips that still make no more items than `strip_rows` does, rounded up to whole
-// waves of resident blocks.  With strips of exactly `strip_rows` rows, 16 members each of 128^2,
-// 256^2 and 512^2 are 168 items of 64 rows or 336 of 32 for 304 resident blocks: 57.6 us a step at the
-// best power of two, 45.1 with 280 items of 40 rows (with noise 77.6 and 65.0).
-// Multiples of 8 rows: the kernel works in whole turns of its ring (ending an item within a turn costs
-// every iteration 15 to 25 %, the unrolled turn being one schedule no longer).
+// The shortest strips, none above `strip_rows` rows, that still make no more items than those of
+// `strip_rows` do, rounded up to whole waves of resident blocks.  With strips of exactly `strip_rows`
+// rows, 16 members each of 128^2, 256^2 and 512^2 are 168 items of 64 rows or 336 of 32 for 304
+// resident blocks: 57.6 us a step at the best power of two, 45.1 with 280 items of 40 rows (with noise
+// 77.6 and 65.0).
+// Shorter ones are multiples of 8 rows: the kernel works in whole turns of its ring (ending an item within
+// a turn costs every iteration 15 to 25 %, the unrolled turn being one schedule no longer).
 int fitted_rows(const pg_sweep* w, int lanes, int strip_rows) {
   const long long resident = static_cast<long long>(lanes_blocks_per_sm(lanes, true)) * w->sm_count;
   int max_ny = 8;
@@ -583,7 +584,8 @@ int fitted_rows(const pg_sweep* w, int lanes, int strip_rows) {
   strip_rows = std::min(strip_rows, max_ny);
   const long long items = count_items(w, lanes, strip_rows);
   const long long limit = (items + resident - 1) / resident * resident;
-  int lo = 1, best = (strip_rows + 7) / 8;  // bisection: the count all but falls with the height
+  int lo = 1, best = strip_rows / 8;  // bisection: the count all but falls with the height
+  if (count_items(w, lanes, 8 * best) > limit) return strip_rows;
   while (lo < best) {
     const int mid = (lo + best) / 2;
     if (count_items(w, lanes, 8 * mid) <= limit)
