@@ -84,14 +84,15 @@ __global__ void __launch_bounds__(MaxThreads<T>::value, 1)
   const bool multi = GENERAL && L > 1;  // several separable lasers: sum the terms per site
   const T hh = dt * T(0.5), h6 = dt / T(6), h3 = dt / T(3);
 
-  // The thread's column of row 0.  The general variants index the arrays themselves, which frees the
-  // registers of the members' pointers (two reservoir fields with noise: 80 -> 56 bytes spilled,
-  // 1024 x 1355 x 2 84.3 -> 77.1 us a step); the plain ones have them to spare (64^2 x 128 12.5 us with
-  // pointers, 13.0 without).
+  // The thread's column of row 0.  The general variants with noise or two reservoir fields index the
+  // arrays themselves, which frees the registers of the members' pointers (two fields with noise:
+  // 80 -> 56 bytes spilled, 1024 x 1355 x 2 84.3 -> 77.1 us a step); the others have them to spare
+  // (64^2 x 128 12.5 us with pointers, 13.0 without; 4096^2 without reservoir or noise 254 and 269).
+  constexpr bool kIndex = GENERAL && (TWO || NOISE);
   const long long first = member * plane;
-  const long long own = (GENERAL ? first : 0) + gx;
-  const C2* psi_m = GENERAL ? psi_in : psi_in + first;
-  const T* n_m = GENERAL ? n_in : n_in + first;
+  const long long own = (kIndex ? first : 0) + gx;
+  const C2* psi_m = kIndex ? psi_in : psi_in + first;
+  const T* n_m = kIndex ? n_in : n_in + first;
   constexpr bool two = GENERAL && TWO;  // a second (inactive) reservoir field
   const long long own2 = own + static_cast<long long>(g.members) * plane;  // in the inactive field
   const T* pump_m = pump + member * g.pump_stride;
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(MaxThreads<T>::value, 1)
         ou = ou < T(0) ? T(0) : ou;
         if (i >= 8 && i - 8 < h_eff && col_writes) {
           const long long o = static_cast<long long>(row_out) * nx;
-          const long long at = GENERAL ? own + o : first + gx + o;
+          const long long at = kIndex ? own + o : first + gx + o;
           if (NOISE) {
             WignerDraw<T>::apply(wz, fma_t(k.noise_b, on, k.noise_a), ore, oim);
           }
