@@ -735,18 +735,22 @@ int wide_rk4_grid(int nx, int ny, int members, int sm_count, int terms) {
   const long long rows = static_cast<long long>(members) * bands * ny;
   const long long blocks = static_cast<long long>(per_sm) * std::max(1, sm_count);
   // Blocks of 16 rows or more, as many as fit.  Where those leave SMs without a block, or are all that fit, rows
-  // of at most 1024 sites go by whole strips of members instead where that leaves the busiest block
-  // fewer rows (one 1024^2 member: 28 us a step with 64 blocks of 16 rows, 20 with 128 of 8; 64 members of 256^2
-  // with a complex potential 82 and 72; between the two, shorter blocks only add fill: 64 members of 128^2
-  // 19.5 us with 512 blocks of 16 rows, 22 with 1024 of 8).
+  // of at most 1024 sites go by whole strips of members instead where those need fewer turns of the
+  // ring (iterations come in whole turns): one 1024^2 member: 28 us a step with 64 blocks of 16 rows, 20 with
+  // 128 of 8; 64 members of 256^2 with a complex potential 82 and 73.  With as many turns the larger grid
+  // stays (four 1024^2 members with a complex potential 72.5 us with 152 blocks, 75.1 with 128); between
+  // the two, shorter blocks only add fill (64 members of 128^2 19.5 us with 512 blocks of 16 rows, 22 with
+  // 1024 of 8).
+  const long long even = std::min(blocks, std::max<long long>(1, rows / 16));
   if (nx <= 1024 && (rows / 16 < sm_count || rows / 16 >= blocks)) {
+    auto turns = [&](long long b) { return (static_cast<long long>(row_iterations(members, ny, b)) + kRing - 1) / kRing; };
     const long long b = row_blocks(members, ny, blocks);
+    if (turns(b) >= turns(even)) return static_cast<int>(even);
     if (b % members != 0) return static_cast<int>(b);
-    // Iterations come in whole turns of the ring: the fewest strips that need as many turns.
-    const long long turn = ((ny + b / members - 1) / (b / members) + 8 + kRing - 1) / kRing * kRing;
-    return static_cast<int>(members * ((ny + turn - 9) / (turn - 8)));
+    // The fewest strips that need as many turns.
+    return static_cast<int>(members * ((ny + kRing * turns(b) - 9) / (kRing * turns(b) - 8)));
   }
-  return static_cast<int>(std::min(blocks, std::max<long long>(1, rows / 16)));
+  return static_cast<int>(even);
 }
 
 cudaError_t launch_rk4_wide(const float* psi_in, const float* n_in, const float* pump,
