@@ -265,18 +265,20 @@ int pg_rk4_get_kernel(pg_solver* s, int32_t* kind);
  * member has a kinetic relaxation term. */
 int pg_rk4_plan(const pg_config* cfg, int32_t relax, int32_t sm_count, int32_t plan[4]);
 
-/* Failure detection of the TMA-fed RK4 kernels (full-width, four-sites-a-thread, cluster
- * form; no counterpart in the reference, whose kernels wait on nothing).  Every wait of these
- * kernels on an mbarrier -- a row copy, the block's row exchange, a neighbouring CTA's edge
- * values -- gives up after 100000 polls, a bound compiled into the kernels.  Once a wait of
- * the thread that feeds a block's row ring has given up, it completes later ring slots without
- * copying into them, so the block's remaining waits pass at once and the kernel ends in about
- * the time of one full wait; copies still in flight are waited for before the block exits.
+/* Failure detection of the RK4 kernels that wait on mbarriers: the full-width kernel, its four-sites-a-
+ * thread and cluster forms, and windows of more than 512 columns with a complex potential (no
+ * counterpart in the reference, whose kernels wait on nothing).  Every such wait -- a row copy, the
+ * block's row exchange, a neighbouring CTA's edge values -- gives up after 100000 polls, a bound compiled
+ * into the full-width kernels.  Once a wait of the thread that feeds a full-width block's row ring has
+ * given up, it completes later ring slots without copying into them, so the block's remaining waits pass
+ * at once and the kernel ends in about the time of one full wait; copies still in flight are waited for
+ * before the block exits.
  * The next pg_synchronize or pg_get_state then returns PG_ERR_TIMEOUT, and the state is
  * invalid until set again.  `polls` is 100000 (the default) or 0, the give-up setting: the
- * kernels withhold each block's first row copy, so that a wait runs out on a healthy GPU and
- * the failure path can be exercised (PG_ERR_INVALID for other values).  Changing it drops the
- * captured CUDA graphs. */
+ * full-width kernels withhold each block's first row copy, so that a wait runs out on a healthy GPU, the
+ * windows do not poll at all, and the failure path can be exercised (PG_ERR_INVALID for other
+ * values).  The streaming and tile kernels and the other windows have no such wait and step as always.
+ * Changing it drops the captured CUDA graphs. */
 int pg_set_wait_limit(pg_solver* s, int32_t polls);
 
 /* CUDA graph capture failures (rk4_cuda_solver.py:3591-3602 restores the pre-chunk state and

@@ -258,6 +258,7 @@ cudaError_t launch_step(pg_solver* s, int from, int step_offset) {
     w.pot_stride = s->cfg.potential_per_member ? s->plane : 0;
     w.pot_kind = f.potential;
     w.relax = f.relax;
+    w.wait_limit = s->wait_limit;
     return pg::launch_rk4_window(static_cast<const float*>(s->psi[from]), static_cast<const float*>(s->res[from]),
                                  static_cast<const float*>(s->pump), static_cast<float*>(s->psi[to]),
                                  static_cast<float*>(s->res[to]),

@@ -55,9 +55,12 @@ __global__ void __launch_bounds__(WindowShape<WMAX>::THREADS, WindowShape<WMAX>:
                       const unsigned long long* __restrict__ step_base, const int step_offset,
                       const float dt, const WindowGeom g, int* __restrict__ err_flag) {
   constexpr int HALF = WMAX / 2;  // exchange-buffer stride
-  // One block an SM: a split arrive/wait barrier lets its warps drift apart by up to a row; several
-  // blocks interleave already, and a block-wide barrier is cheaper.
-  constexpr bool kSplit = WindowShape<WMAX>::BLOCKS == 1;
+  // Rows meet at a block-wide barrier, but for one block an SM with a complex potential: its loads from
+  // global memory stall the warps unevenly, and a split arrive/wait barrier lets them drift apart by up to
+  // a row (8 x 1020^2 125 us a step against 138; without a potential 63 against 59).  Each warp arrives once: an
+  // arrival of all its lanes counts as 32 at once, and where a wait had given up, more arrivals than a phase
+  // still expects, which is an error of the barrier; one at a time they only move on to the next phase.
+  constexpr bool kSplit = WindowShape<WMAX>::BLOCKS == 1 && POT == 2 && TERMS == 1;
   if (g.halt != nullptr && __ldcg(g.halt) != 0) return;  // steady-state monitor halted the run
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float2* ring_psi = reinterpret_cast<float2*>(smem_raw);                 // [kWinRing][WMAX]
@@ -87,7 +90,7 @@ __global__ void __launch_bounds__(WindowShape<WMAX>::THREADS, WindowShape<WMAX>:
   const long long plane = static_cast<long long>(nx) * ny;
 
   if (kSplit && t == 0) {
-    mbar_init(xbar, blockDim.x);
+    mbar_init(xbar, blockDim.x / 32);
     fence_mbar_init();
   }
 
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(WindowShape<WMAX>::THREADS, WindowShape<WMAX>:
           // Every thread has arrived at the end of iteration i-1: published its stage values there
           // and finished every read of iteration i-1.
           const unsigned gi = it + i;
-          if (gi > 0 && !mbar_wait_bounded(xbar, (gi - 1) & 1u, kWaitPolls)) timed_out = true;
+          if (gi > 0 && !mbar_wait_bounded(xbar, (gi - 1) & 1u, g.wait_limit)) timed_out = true;
         }
         // Row r+3 into the slot of row r-5, whose last reader was this thread's stage 4.
         if (i + 3 < n_iter) issue((j + 3) % 8);
@@ -364,10 +367,12 @@ __global__ void __launch_bounds__(WindowShape<WMAX>::THREADS, WindowShape<WMAX>:
         }
         row_out = row_out + 1 == ny ? 0 : row_out + 1;
         cp_async_wait<2>();  // row r + 1 has landed
-        if (kSplit)
-          mbar_arrive(xbar);
-        else
+        if (kSplit) {
+          __syncwarp();
+          if ((t & 31) == 0) mbar_arrive(xbar);
+        } else {
           __syncthreads();
+        }
       }
     }
     it += n_iter;

@@ -20,6 +20,7 @@ struct WindowGeom {
   long long pot_stride;
   int pot_kind;
   int relax;
+  int wait_limit;          // polls of a wait on the split barrier, before it gives up
 };
 
 // The kernel a grid is stepped with when the caller leaves the choice, and the geometry of each

@@ -244,9 +244,10 @@ class RK4Engine:
         return int(h.value), int(w.value)
 
     def set_wait_limit(self, polls):
-        """100000 (the default: the polls each mbarrier wait of the TMA-fed kernels makes before it
-        gives up) or 0: the kernels withhold each block's first row copy, so that a wait runs
-        out on a healthy GPU and the next synchronising call reports PG_ERR_TIMEOUT."""
+        """100000 (the default: the polls each mbarrier wait of an RK4 kernel makes before it gives up)
+        or 0: in the kernels that have such waits (the full-width ones, windows of more than 512
+        columns with a complex potential) a wait then gives up on a healthy GPU, and the next
+        synchronising call reports PG_ERR_TIMEOUT."""
         _lib.check(self.lib.pg_set_wait_limit(self.handle, int(polls)), "pg_set_wait_limit")
 
     def kernel(self) -> int:
