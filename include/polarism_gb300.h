@@ -262,8 +262,8 @@ int pg_rk4_get_kernel(pg_solver* s, int32_t* kind);
 /* The automatic choice for a configuration on a GPU of `sm_count` SMs (0: 152), without one: plan[0] the
  * kernel as pg_rk4_get_kernel reports it; then the streaming kernel's tile width and strip height, or
  * the tile shape's index, or the window's capacity in columns, its bands a row and its blocks.  `relax`: a
- * member has a kinetic relaxation term. */
-int pg_rk4_plan(const pg_config* cfg, int32_t relax, int32_t sm_count, int32_t plan[4]);
+ * member has a kinetic relaxation term; `noise`: pg_set_noise turned the noise on. */
+int pg_rk4_plan(const pg_config* cfg, int32_t relax, int32_t noise, int32_t sm_count, int32_t plan[4]);
 
 /* Failure detection of the RK4 kernels that wait on mbarriers: the full-width kernel, its four-sites-a-
  * thread and cluster forms, and windows of more than 512 columns with a complex potential (no

@@ -90,7 +90,7 @@ SIGNATURES = {
     "pg_field_norms": (C.c_int, [_vp, _i32, _i32, _i64, _f64, _vp, _vp]),
     "pg_field_norms_noalloc": (C.c_int, [_vp, _i32, _i32, _i64, _f64, _vp, _vp]),
     "pg_rk4_set_kernel": (C.c_int, [_vp, _i32]),
-    "pg_rk4_plan": (C.c_int, [C.POINTER(PgConfig), _i32, _i32, C.POINTER(_i32)]),
+    "pg_rk4_plan": (C.c_int, [C.POINTER(PgConfig), _i32, _i32, _i32, C.POINTER(_i32)]),
     "pg_rk4_get_kernel": (C.c_int, [_vp, C.POINTER(_i32)]),
     "pg_set_wait_limit": (C.c_int, [_vp, _i32]),
     "pg_test_fail_next_graph": (C.c_int, [_vp, _i32]),

@@ -472,7 +472,7 @@ int pg_create(const pg_config* cfg, const pg_physics* physics, pg_solver** out) 
     if ((e = cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming)) != cudaSuccess)
       return fail(e, "staging event");
   }
-  s->plan = pg::plan_rk4(*cfg, features(s), s->sm_count);
+  s->plan = pg::plan_rk4(*cfg, features(s), s->noise, s->sm_count);
   s->geom = s->plan.stream;
   int rc = upload_consts(s);
   if (rc != PG_OK) {
@@ -613,7 +613,7 @@ int pg_rk4_prepare(pg_solver* s, int32_t n_steps) {
   return PG_OK;
 }
 
-int pg_rk4_plan(const pg_config* cfg, int32_t relax, int32_t sm_count, int32_t plan[4]) {
+int pg_rk4_plan(const pg_config* cfg, int32_t relax, int32_t noise, int32_t sm_count, int32_t plan[4]) {
   PG_CHECK(cfg && plan && cfg->nx >= 4 && cfg->ny >= 4 && cfg->members >= 1, PG_ERR_INVALID,
            "pg_rk4_plan: bad argument");
   pg::RK4Features f{};
@@ -621,7 +621,7 @@ int pg_rk4_plan(const pg_config* cfg, int32_t relax, int32_t sm_count, int32_t p
   f.reservoir = cfg->reservoir;
   f.pump_terms = std::max(1, cfg->pump_terms);
   f.relax = relax ? 1 : 0;
-  const pg::RK4Plan p = pg::plan_rk4(*cfg, f, sm_count);
+  const pg::RK4Plan p = pg::plan_rk4(*cfg, f, noise != 0, sm_count);
   plan[1] = plan[2] = plan[3] = 0;
   switch (p.route) {
     case pg::RK4Route::kStream:
@@ -698,6 +698,7 @@ int pg_set_noise(pg_solver* s, const uint64_t* seeds, const double* gamma, const
     s->dt_over_4dv = dt_over_4dv;
     s->noise = true;
   }
+  s->plan = pg::plan_rk4(s->cfg, features(s), s->noise, s->sm_count);  // which kernel is ahead depends on it
   free_graphs(s);
   int rc = upload_consts(s);
   if (rc != PG_OK) return rc;

@@ -713,6 +713,32 @@ cudaError_t configure_wide_rk4() {
   return e;
 }
 
+int wide_rk4_blocks(int nx, int ny, int members, int per_sm, int sm_count) {
+  // Rows wider than 1024 sites (BAND) are separate 1024-site bands, each its own row stream.
+  const long long bands = nx > 1024 ? nx / 1024 : 1;
+  const long long rows = static_cast<long long>(members) * bands * ny;
+  const long long blocks = static_cast<long long>(per_sm) * std::max(1, sm_count);
+  // Blocks of 16 rows or more, as many as fit.  Where those leave SMs without a block, or are all that fit, rows
+  // of at most 1024 sites go by whole strips of members instead where those need fewer turns of the
+  // ring (iterations come in whole turns): one 1024^2 member: 28 us a step with 64 blocks of 16 rows, 20 with
+  // 128 of 8; 64 members of 256^2 with a complex potential 82 and 73.  With as many turns the larger grid
+  // stays (four 1024^2 members with a complex potential 72.5 us with 152 blocks, 75.1 with 128) unless its
+  // blocks cross from member to member (eighty 512 x 77 with two lasers 68.5 us with 304 blocks, 54.1 with
+  // 240); between the two, shorter blocks only add fill (64 members of 128^2 19.5 us with 512 blocks of
+  // 16 rows, 22 with 1024 of 8).
+  const long long even = std::min(blocks, std::max<long long>(1, rows / 16));
+  if (nx <= 1024 && (rows / 16 < sm_count || rows / 16 >= blocks)) {
+    auto turns = [&](long long b) { return (static_cast<long long>(row_iterations(members, ny, b)) + kRing - 1) / kRing; };
+    const long long b = row_blocks(members, ny, blocks);
+    const bool whole = b % members == 0, crosses = even % members != 0;
+    if (turns(b) > turns(even) || (turns(b) == turns(even) && !(whole && crosses))) return static_cast<int>(even);
+    if (!whole) return static_cast<int>(b);
+    // The fewest strips that need as many turns.
+    return static_cast<int>(members * ((ny + kRing * turns(b) - 9) / (kRing * turns(b) - 8)));
+  }
+  return static_cast<int>(even);
+}
+
 int wide_rk4_grid(int nx, int ny, int members, int sm_count, int terms) {
   if (use_cluster(nx)) {
     // Whole clusters, as many as fit at once, and at least 16 rows a cluster.
@@ -730,27 +756,7 @@ int wide_rk4_grid(int nx, int ny, int members, int sm_count, int terms) {
     case 1024: per_sm = blocks_shape<1024, false>(true, terms); break;
     default: per_sm = blocks_shape<1024, true>(true); break;
   }
-  // Rows wider than 1024 sites (BAND) are separate 1024-site bands, each its own row stream.
-  const long long bands = nx > 1024 ? nx / 1024 : 1;
-  const long long rows = static_cast<long long>(members) * bands * ny;
-  const long long blocks = static_cast<long long>(per_sm) * std::max(1, sm_count);
-  // Blocks of 16 rows or more, as many as fit.  Where those leave SMs without a block, or are all that fit, rows
-  // of at most 1024 sites go by whole strips of members instead where those need fewer turns of the
-  // ring (iterations come in whole turns): one 1024^2 member: 28 us a step with 64 blocks of 16 rows, 20 with
-  // 128 of 8; 64 members of 256^2 with a complex potential 82 and 73.  With as many turns the larger grid
-  // stays (four 1024^2 members with a complex potential 72.5 us with 152 blocks, 75.1 with 128); between
-  // the two, shorter blocks only add fill (64 members of 128^2 19.5 us with 512 blocks of 16 rows, 22 with
-  // 1024 of 8).
-  const long long even = std::min(blocks, std::max<long long>(1, rows / 16));
-  if (nx <= 1024 && (rows / 16 < sm_count || rows / 16 >= blocks)) {
-    auto turns = [&](long long b) { return (static_cast<long long>(row_iterations(members, ny, b)) + kRing - 1) / kRing; };
-    const long long b = row_blocks(members, ny, blocks);
-    if (turns(b) >= turns(even)) return static_cast<int>(even);
-    if (b % members != 0) return static_cast<int>(b);
-    // The fewest strips that need as many turns.
-    return static_cast<int>(members * ((ny + kRing * turns(b) - 9) / (kRing * turns(b) - 8)));
-  }
-  return static_cast<int>(even);
+  return wide_rk4_blocks(nx, ny, members, per_sm, sm_count);
 }
 
 cudaError_t launch_rk4_wide(const float* psi_in, const float* n_in, const float* pump,

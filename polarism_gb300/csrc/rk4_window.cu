@@ -28,9 +28,8 @@ long long row_blocks(long long units, int ny, long long slots) {
 // iterations; an iteration of an SM with W resident warps takes max(0.68, 0.36 + 0.056 W) us: the
 // dependency chain of one thread, or issue slots (measured with Wigner noise on grids from 256^2
 // to 4096^2, windows of 3 to 16 warps, one to four blocks an SM: 0.66-0.73 us with 3 to 6 warps,
-// 0.79-0.97 with 8 to 10, 1.02-1.1 with 12, 1.2-1.3 with 16).  Returns the modelled time of a step in
-// us, without the launch; negative where no window of these capacities takes the row.
-double choose_rk4_window(int nx, int ny, int members, int sm_count, WindowGeom* g) {
+// 0.79-0.97 with 8 to 10, 1.02-1.1 with 12, 1.2-1.3 with 16).  False where no window of these capacities takes the row.
+bool choose_rk4_window(int nx, int ny, int members, int sm_count, WindowGeom* g) {
   const int sms = sm_count > 0 ? sm_count : 152;
   const int capacity[] = {256, 320, 512, 1024};
   double best = -1.0;
@@ -67,7 +66,7 @@ double choose_rk4_window(int nx, int ny, int members, int sm_count, WindowGeom* 
   g->nx = nx;
   g->ny = ny;
   g->members = members;
-  return best;
+  return best >= 0.0;
 }
 
 cudaError_t launch_rk4_window(const float* psi_in, const float* n_in, const float* pump, float* psi_out,

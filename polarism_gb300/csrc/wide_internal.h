@@ -29,6 +29,8 @@ size_t wide_rk4_smem(int nx);
 cudaError_t configure_wide_rk4();
 // Grid of the full-width kernel for this shape: persistent blocks (or, for rows of 2048 to
 // 8192 sites, whole clusters of nx / 1024 CTAs), at least 16 rows of work each.
+// Blocks of its rows of other widths with `per_sm` resident blocks an SM.
+int wide_rk4_blocks(int nx, int ny, int members, int per_sm, int sm_count);
 int wide_rk4_grid(int nx, int ny, int members, int sm_count, int terms = 1);
 cudaError_t launch_rk4_wide(const float* psi_in, const float* n_in, const float* pump,
                             float* psi_out, float* n_out, const RhsConst<float>* consts,

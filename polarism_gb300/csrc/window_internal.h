@@ -31,13 +31,13 @@ struct RK4Plan {
   WindowGeom window{};  // FP32
   int tile = 0;         // tile shape of rk4_tile_f32.cu / rk4_tile_f64.cu
 };
-RK4Plan plan_rk4(const pg_config& cfg, const RK4Features& f, int sm_count);
+RK4Plan plan_rk4(const pg_config& cfg, const RK4Features& f, bool noise, int sm_count);
 
 double row_iterations(long long units, int ny, long long blocks);
 long long row_blocks(long long units, int ny, long long slots);
-// Picks bands, band_w, wmax and blocks for a grid; the modelled time in us, negative if no window holds
-// it (rows beyond some 500,000 sites).
-double choose_rk4_window(int nx, int ny, int members, int sm_count, WindowGeom* g);
+// Picks bands, band_w, wmax and blocks for a grid; false if no window holds it (rows beyond some 500,000
+// sites).
+bool choose_rk4_window(int nx, int ny, int members, int sm_count, WindowGeom* g);
 cudaError_t launch_rk4_window(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
                               float* n_out, const RhsConst<float>* consts, const float* scales,
                               const unsigned long long* step_base, int step_offset, float dt, bool noise,

@@ -13,14 +13,14 @@ def plan():
 
     lib = _lib.load(build.build())
 
-    def ask(nx, ny, members, precision="single", reservoir="single", potential=0, lasers=1, eta=False, sms=152):
+    def ask(nx, ny, members, precision="single", reservoir="single", potential=0, lasers=1, eta=False, noise=False, sms=152):
         cfg = _lib.PgConfig(nx=nx, ny=ny, members=members,
                             precision=_lib.PG_SINGLE if precision == "single" else _lib.PG_DOUBLE,
                             reservoir={"none": 0, "single": 1, "double": 2, "quadratic-double": 3}[reservoir],
                             potential=potential, dx=1.0, dy=1.0, dt=1e-3, components=1, reservoir_components=1,
                             pump_terms=lasers)
         out = (C.c_int32 * 4)()
-        _lib.check(lib.pg_rk4_plan(C.byref(cfg), int(eta), sms, out), "pg_rk4_plan")
+        _lib.check(lib.pg_rk4_plan(C.byref(cfg), int(eta), int(noise), sms, out), "pg_rk4_plan")
         return list(out)
 
     return ask
@@ -52,3 +52,22 @@ def test_more_members_than_a_launch_holds(plan):
     assert plan(128, 4, 70000)[0] in (WIDE, WINDOW)
     assert plan(100, 60, 100000)[0] == WINDOW
     assert plan(128, 4, 70000, reservoir="double")[0] == STREAM  # no kernel takes it: refused at the launch
+
+
+@pytest.mark.parametrize("grid,options,noise,kernels", [
+    # us a step of the kernels named against the ones that an estimate without the noise, the number of
+    # schedulers or the crossings between members took
+    ((128, 128, 128), {}, False, (WINDOW,)),                                 # 21.0; streaming 24.2
+    ((64, 64, 64), {}, False, (STREAM,)),                                    # 7.9; tiles 8.9
+    ((128, 128, 96), dict(potential=2), False, (WIDE,)),                     # 33.2; windows 39.0
+    ((128, 128, 96), dict(potential=2), True, (WIDE,)),                      # 35.2; windows 42.9
+    ((100, 100, 64), dict(potential=2), True, (STREAM,)),                    # 25.9; windows 32.7
+    ((64, 64, 772), dict(eta=True), True, (STREAM,)),                        # 66.8; windows 102
+    ((64, 64, 512), dict(lasers=2), True, (STREAM,)),                        # 74.8; windows 100
+    ((64, 64, 1279), dict(lasers=2), False, (STREAM,)),                      # 140; windows 185
+    ((600, 500, 6), dict(reservoir="double"), False, (STREAM,)),             # 65; tiles 77
+    ((3000, 100, 2), dict(reservoir="none"), False, (STREAM,)),              # 23.6; tiles 27.9
+    ((200, 200, 32), dict(potential=2), False, (WINDOW,)),                   # 30.9; streaming 47.9
+    ((256, 256, 1), dict(lasers=2), False, (TILE,))])                        # 8.3; windows 9.6
+def test_choice_follows_what_was_measured(plan, grid, options, noise, kernels):
+    assert plan(*grid, noise=noise, **options)[0] in kernels

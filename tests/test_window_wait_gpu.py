@@ -43,7 +43,7 @@ def test_zero_poll_limit_reports_timeout_and_solver_recovers(cuda_lib, nx, ny, m
                         dy=0.4, dt=5e-4, components=1, reservoir_components=1, pump_terms=1)
     plan = (C.c_int32 * 4)()
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    _lib.check(cuda_lib.pg_rk4_plan(C.byref(cfg), 0, sms, plan), "pg_rk4_plan")
+    _lib.check(cuda_lib.pg_rk4_plan(C.byref(cfg), 0, 0, sms, plan), "pg_rk4_plan")
     assert list(plan)[:3] == [5, 1024, bands]  # the capacity that has the split barrier
     eng = make()
     assert eng.kernel() == 5
