@@ -15,9 +15,10 @@ __device__ __forceinline__ float mul_rn_t(float a, float b) { return __fmul_rn(a
 __device__ __forceinline__ double mul_rn_t(double a, double b) { return __dmul_rn(a, b); }
 
 // psi (1 + dx) (1 + dy) scale, with the factor differences d stored in place of the factors (see
-// setup_tables) and scale a power of two.  FP32 forms the combined difference first, so that
-// psi is rounded once; FP64, bound by its arithmetic, takes two products psi + psi d (10 instead of
-// 16 instructions).
+// setup_tables) and scale a power of two; psi is rounded once.  FP32 forms the combined difference first.
+// FP64, bound by its arithmetic, adds both small terms to psi together, psi + (t + (psi + t) dy) with
+// t = psi dx: 14 instructions instead of 16, and at phases below a radian the combined form's error
+// (4.7e-17 rms a kick; two products psi + psi d, as many instructions, round psi twice: 6.7e-17).
 __device__ __forceinline__ float2 kick(float2 v, float2 dx, float2 dy, float scale) {
   const float2 dxy = cmul(dx, dy);
   const float2 f1 = make_float2(dx.x + dy.x + dxy.x, dx.y + dy.y + dxy.y);
@@ -25,9 +26,10 @@ __device__ __forceinline__ float2 kick(float2 v, float2 dx, float2 dy, float sca
   return make_float2((v.x + vf.x) * scale, (v.y + vf.y) * scale);
 }
 __device__ __forceinline__ double2 kick(double2 v, double2 dx, double2 dy, double scale) {
-  const double2 a = make_double2(v.x + (v.x * dx.x - v.y * dx.y), v.y + (v.x * dx.y + v.y * dx.x));
-  return make_double2((a.x + (a.x * dy.x - a.y * dy.y)) * scale,
-                      (a.y + (a.x * dy.y + a.y * dy.x)) * scale);
+  const double2 t = make_double2(fma(v.x, dx.x, -(v.y * dx.y)), fma(v.x, dx.y, v.y * dx.x));
+  const double2 a = make_double2(v.x + t.x, v.y + t.y);
+  return make_double2((v.x + fma(a.x, dy.x, fma(-a.y, dy.y, t.x))) * scale,
+                      (v.y + fma(a.x, dy.y, fma(a.y, dy.x, t.y))) * scale);
 }
 
 // Midpoint RK2 reservoir half step at frozen |psi|^2 with the final clamp
