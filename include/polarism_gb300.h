@@ -402,9 +402,12 @@ int pg_fno_sum_slices(const float* parts, float* out, int64_t n, int32_t count, 
                       void* stream);
 /* GEMM engine: 0 = tcgen05.mma with FP32 accumulators in tensor memory (default), 1 = mma.sync
  * (the pre-Blackwell tensor-core path, kept as the cross-check).  pg_gemm_timeouts reports
- * (and optionally clears) whether a tcgen05 GEMM's bounded completion wait gave up; its
- * results are then invalid. */
+ * (and optionally clears) whether a tcgen05 kernel's bounded completion wait gave up; its
+ * results are then invalid.  pg_gemm_set_wait_limit: polls of the fused passes' waits, 200000 (the
+ * default) or 0, the give-up setting: every wait gives up at once, so that the failure path can be
+ * exercised on a healthy GPU (PG_ERR_INVALID for other values).  Both settings are the process's. */
 int pg_gemm_set_engine(int32_t engine);
+int pg_gemm_set_wait_limit(int32_t polls);
 int pg_gemm_timeouts(int32_t* count, int32_t clear);
 /* y = bf16(x) (round to nearest even). */
 int pg_fno_to_bf16(const float* x, void* y, int64_t n, void* stream);

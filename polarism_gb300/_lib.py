@@ -132,6 +132,7 @@ SIGNATURES = {
                                   _i64, _vp]),
     "pg_fno_sum_slices": (C.c_int, [_vp, _vp, _i64, _i32, _i32, _vp]),
     "pg_gemm_set_engine": (C.c_int, [_i32]),
+    "pg_gemm_set_wait_limit": (C.c_int, [_i32]),
     "pg_gemm_timeouts": (C.c_int, [C.POINTER(_i32), _i32]),
     "pg_fno_to_bf16": (C.c_int, [_vp, _vp, _i64, _vp]),
     "pg_fno_bias_act": (C.c_int, [_vp, _vp, _vp, _vp, _i32, _i64, _i64, _i32, _vp]),

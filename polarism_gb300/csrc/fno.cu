@@ -170,8 +170,6 @@ constexpr int kTcSmemA = kTcM * kTcK * 2;                // 16 KB
 constexpr int kTcSmemB = kTcN * kTcK * 2;                // 8 KB
 // 28 KB per CTA keeps at most 8 CTAs (8 x 64 TMEM columns = 512) on an SM.
 constexpr int kTcSmem = 28 * 1024;
-constexpr int kTcWaitLimit = 200000;
-
 // kind::f16 instruction descriptor: D = F32, A = B = BF16, both K-major, N = 64, M = 128.
 constexpr uint32_t kTcIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kTcN >> 3) << 17) |
                               (static_cast<uint32_t>(kTcM >> 4) << 24);
@@ -704,6 +702,7 @@ __global__ void mse_kernel(const float* __restrict__ pred, const float* __restri
 
 __device__ int g_gemm_timeouts = 0;  // set when a bounded wait of a tcgen05 kernel gave up
 int g_gemm_engine = 0;                // 0: tcgen05 (default), 1: mma.sync
+int g_gemm_wait_limit = kTcWaitLimit;
 
 int grid_for(long long n) {
   const long long b = (n + 255) / 256;
@@ -717,6 +716,7 @@ cudaError_t gemm_timeout_flag(int** flag) {
 }
 
 int gemm_engine() { return g_gemm_engine; }
+int gemm_wait_limit() { return g_gemm_wait_limit; }
 
 }  // namespace pg
 
@@ -777,6 +777,13 @@ int pg_gemm_set_engine(int32_t engine) {
   PG_CHECK(engine == 0 || engine == 1, PG_ERR_INVALID,
            "pg_gemm_set_engine: 0 (tcgen05 tensor cores) or 1 (mma.sync)");
   pg::g_gemm_engine = engine;
+  return PG_OK;
+}
+
+int pg_gemm_set_wait_limit(int32_t polls) {
+  PG_CHECK(polls == 0 || polls == pg::kTcWaitLimit, PG_ERR_INVALID,
+           "pg_gemm_set_wait_limit: polls must be 0 (every wait gives up at once) or 200000 (the default)");
+  pg::g_gemm_wait_limit = polls;
   return PG_OK;
 }
 

@@ -128,6 +128,7 @@ struct LayerArgs {
   int w_t, table_rows, cin, cout, n, B, k2;
   int o_t, o_v, o_z, o_bar, cols;  // shared-memory offsets (w at 0) and TMEM columns
   int v_bytes, z_bytes;            // of one of the two buffers
+  int waits;                       // 0: the give-up setting, every completion wait has failed
 };
 
 // x[b, co, p] = sum_k w[co, k] v[b, k, p] + sum_q z[b, co, y, q] table[q, x] + bias[co] for the pixels
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(kThreads, kLayerBlocks) layer_kernel(const Lay
   };
 
   const int rows = g.B * g.n;
-  bool ok = true;
+  bool ok = g.waits != 0;
   uint32_t phase = 0;
   int buf = 0;
   if (static_cast<int>(blockIdx.x) < rows) load(blockIdx.x, 0);
@@ -265,7 +266,7 @@ struct OuterArgs {
   const bf16* x;  // [B][cin][plane]
   float* parts;   // [B * slices][cout][cin]
   long long plane;
-  int cout, cin, chunk, slices, cols, slack;
+  int cout, cin, chunk, slices, cols, waits;
 };
 
 // parts[b, s] = sum over the `chunk` sites of slice s of g[b, :, p] x[b, :, p]^T: both operands K-major as they
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(kOuterThreads) outer_kernel(const OuterArgs g,
   };
   for (int i = 0; i < STAGES - LAG; ++i) load(i);
   const uint32_t idesc = tc_idesc(np, false, false);
-  bool ok = true;
+  bool ok = g.waits != 0;
   for (int i = 0; i < slabs; ++i) {
     cp_async_wait<STAGES - LAG - 1>();
     fence_async_proxy();
@@ -358,7 +359,7 @@ struct DftYArgs {
   const bf16* s;    // [batch][K][m2], columns re | im
   float* out;       // [batch][M][m2] or null
   bf16* out_bf;
-  int n, m2, K, M, cols, o_s, o_bar;
+  int n, m2, K, M, cols, o_s, o_bar, waits;
   float sign;       // of gim's product in the real part
 };
 
@@ -409,7 +410,7 @@ __global__ void __launch_bounds__(kThreads) dft_y_kernel(const DftYArgs g, int* 
     }
     tc_commit(smem_u32(mbar));
   }
-  const bool ok = mbar_wait_bounded(smem_u32(mbar), 0u, kTcWaitLimit);
+  const bool ok = g.waits && mbar_wait_bounded(smem_u32(mbar), 0u, kTcWaitLimit);
   tc_fence_after();
   const uint32_t lane = tmem + (static_cast<uint32_t>(warp * 32) << 16);
   const int m = g.m2 / 2;
@@ -447,7 +448,7 @@ struct DftXArgs {
   const bf16* table;  // [n][m2], or [m2][n] when table_rows
   bf16* out;          // [rows][m2]
   long long rows;
-  int n, m2, table_rows, cols, o_b, o_bar;
+  int n, m2, table_rows, cols, o_b, o_bar, waits;
 };
 
 // out = v T, rounded to BF16: 128 rows a block, all of their n values in flight at once, and a second
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(kThreads) dft_x_kernel(const DftXArgs g, int* 
              tc_smem_desc(b + 2 * s * b_group, b_group, g.table_rows ? 128 : kMnChunk), idesc, s > 0);
     tc_commit(smem_u32(mbar));
   }
-  const bool ok = mbar_wait_bounded(smem_u32(mbar), 0u, kTcWaitLimit);
+  const bool ok = g.waits && mbar_wait_bounded(smem_u32(mbar), 0u, kTcWaitLimit);
   tc_fence_after();
   const uint32_t lane = tmem + (static_cast<uint32_t>(warp * 32) << 16);
   bf16* dst = g.out + (r0 + tid) * g.m2;
@@ -626,6 +627,7 @@ int pg_fno_layer(const void* w, int32_t w_transposed, const void* v, const void*
   a.n = n;
   a.B = B;
   a.k2 = modes2;
+  a.waits = pg::gemm_wait_limit() > 0;
   const int smem = pg::layer_geometry(&a);
   PG_CHECK(smem <= pg::kMaxSmem && a.cols <= 512, PG_ERR_UNSUPPORTED, "pg_fno_layer: does not fit an SM");
   int* flag = nullptr;
@@ -659,6 +661,7 @@ int pg_fno_outer(const void* g, const void* x, float* parts, int32_t B, int32_t 
   a.slices = slices;
   a.chunk = static_cast<int>(plane / slices);
   a.cols = pg::tmem_cols(pg::pad16(cin));
+  a.waits = pg::gemm_wait_limit() > 0;
   int* flag = nullptr;
   PG_CUDA(pg::gemm_timeout_flag(&flag));
   const int stage = pg::outer_bytes(cout, cin);  // of 128 sites
@@ -701,6 +704,7 @@ int pg_fno_dft_y(const void* gre, const void* gim, const void* s, float* out, vo
   a.K = inverse ? 2 * modes : n;
   a.M = inverse ? n : 2 * modes;
   a.sign = inverse ? 1.f : -1.f;
+  a.waits = pg::gemm_wait_limit() > 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return inverse ? pg::run_dft_y<true>(a, batch, st) : pg::run_dft_y<false>(a, batch, st);
 }
@@ -720,6 +724,7 @@ int pg_fno_dft_x(const void* v, const void* table, int32_t table_rows, void* out
   a.n = n;
   a.m2 = 2 * modes;
   a.table_rows = table_rows ? 1 : 0;
+  a.waits = pg::gemm_wait_limit() > 0;
   const int smem = pg::dft_x_geometry(&a);
   PG_CHECK(smem <= pg::kMaxSmem, PG_ERR_UNSUPPORTED, "pg_fno_dft_x: does not fit shared memory");
   int* flag = nullptr;

@@ -8,6 +8,9 @@ namespace pg {
 cudaError_t gemm_timeout_flag(int** flag);
 // 0: tcgen05, 1: mma.sync (pg_gemm_set_engine).
 int gemm_engine();
+// Polls of a fused kernel's completion waits, 0 for the give-up setting (pg_gemm_set_wait_limit).  The bound
+// itself is compiled in: read from the arguments it made a training pass 2 % slower.
+int gemm_wait_limit();
 
 // Shared memory of a block at most.
 constexpr int kMaxSmem = 227 * 1024;
