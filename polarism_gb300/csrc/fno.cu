@@ -501,18 +501,20 @@ constexpr size_t kMixSmem = 200 * 1024;
 // The fused multiply-adds are spelled out: one rounding more or less in a spectral value moves the BF16
 // rounding of the operands after it.
 struct MixStage {
-  int samples;    // gathered at a time
+  int samples;    // gathered at a time; 0: not even one fits, the values are read where they lie
   int weights;    // the mode's weights too (they fit)
   size_t bytes;
 };
 
 MixStage mix_stage(int values_per_sample, long long weights, int B) {
   MixStage m{};
+  if (8LL * values_per_sample > static_cast<long long>(kMixSmem)) return m;
   const long long fit = static_cast<long long>(kMixSmem / 2) / (8LL * values_per_sample);
   m.samples = static_cast<int>(fit < 1 ? 1 : fit < kMixSamples ? fit : kMixSamples);
   if (m.samples > B) m.samples = B;
   m.bytes = static_cast<size_t>(m.samples) * values_per_sample * 8;
-  m.weights = weights * 4 <= static_cast<long long>(kMixSmem / 2);
+  m.weights = weights * 4 <= static_cast<long long>(kMixSmem / 2) &&
+              static_cast<long long>(m.bytes) + weights * 4 <= static_cast<long long>(kMixSmem);
   if (m.weights) m.bytes += static_cast<size_t>(weights) * 4;
   return m;
 }
@@ -539,7 +541,7 @@ __device__ __forceinline__ void put_mode(float* out, __nv_bfloat16* out_bf, long
 
 // out[b, o] = sum_i y[b, i] W[i, o], or with ADJOINT dY[b, i] = sum_o dO[b, o] conj(W[i, o]); n_in and n_out
 // are the channels summed over and written.  out and out_bf: either may be null.
-template <bool ADJOINT>
+template <bool ADJOINT, bool STAGED>
 __global__ void __launch_bounds__(256)
     mode_mix_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ wre,
                     const __nv_bfloat16* __restrict__ wim, float* __restrict__ out, __nv_bfloat16* __restrict__ out_bf,
@@ -562,25 +564,30 @@ __global__ void __launch_bounds__(256)
     re_w = sw;
     im_w = sw + weights / len * pitch;
   }
-  for (int b0 = 0; b0 < B; b0 += st.samples) {
-    const int nb = min(st.samples, B - b0);
-    if (b0) __syncthreads();
-    gather_mode(vals, x + static_cast<long long>(b0) * n_in * (4 * m * m), nb * n_in, m, at);
-    __syncthreads();
+  for (int b0 = 0; b0 < B; b0 += STAGED ? st.samples : B) {
+    const int nb = STAGED ? min(st.samples, B - b0) : B;
+    if (STAGED) {
+      if (b0) __syncthreads();
+      gather_mode(vals, x + static_cast<long long>(b0) * n_in * (4 * m * m), nb * n_in, m, at);
+      __syncthreads();
+    }
     for (int t = threadIdx.x; t < nb * n_out; t += blockDim.x) {
       const int c = t % n_out, b = t / n_out;
       const float2* v = vals + b * n_in;
+      const float* src = x + static_cast<long long>(b) * n_in * (4 * m * m) + at;
       float re = 0.f, im = 0.f;
 #pragma unroll 4
       for (int k = 0; k < n_in; ++k) {
         const int w = ADJOINT ? c * pitch + k : k * pitch + c;
         const float r = __bfloat162float(re_w[w]), s = __bfloat162float(im_w[w]);
+        const long long o = static_cast<long long>(k) * (4 * m * m);
+        const float2 value = STAGED ? v[k] : make_float2(src[o], src[o + m]);
         if (ADJOINT) {
-          const float gr = v[k].x, gi = v[k].y;
+          const float gr = value.x, gi = value.y;
           re += __fmaf_rn(gr, r, __fmul_rn(gi, s));
           im += __fmaf_rn(gi, r, -__fmul_rn(gr, s));
         } else {
-          const float a = v[k].x, c2 = v[k].y;
+          const float a = value.x, c2 = value.y;
           re += __fmaf_rn(a, r, -__fmul_rn(c2, s));
           im += __fmaf_rn(c2, r, __fmul_rn(a, s));
         }
@@ -591,6 +598,7 @@ __global__ void __launch_bounds__(256)
 }
 
 // dW[i, o] = sum_b conj(Y[b, i]) dO[b, o] per mode (overwrites).
+template <bool STAGED>
 __global__ void __launch_bounds__(256) mode_mix_back_weight_kernel(const float* __restrict__ y,
                                                                    const float* __restrict__ dout,
                                                                    float* __restrict__ dwre, float* __restrict__ dwim,
@@ -600,17 +608,24 @@ __global__ void __launch_bounds__(256) mode_mix_back_weight_kernel(const float* 
   float2* gs = vals + samples * cin;
   const int at = static_cast<int>(blockIdx.x / m) * 2 * m + static_cast<int>(blockIdx.x % m);
   const long long wbase = static_cast<long long>(blockIdx.x) * cin * cout;
-  for (int b0 = 0; b0 < B; b0 += samples) {
-    const int nb = min(samples, B - b0);
-    if (b0) __syncthreads();
-    gather_mode(ys, y + static_cast<long long>(b0) * cin * (4 * m * m), nb * cin, m, at);
-    gather_mode(gs, dout + static_cast<long long>(b0) * cout * (4 * m * m), nb * cout, m, at);
-    __syncthreads();
+  for (int b0 = 0; b0 < B; b0 += STAGED ? samples : B) {
+    const int nb = STAGED ? min(samples, B - b0) : B;
+    if (STAGED) {
+      if (b0) __syncthreads();
+      gather_mode(ys, y + static_cast<long long>(b0) * cin * (4 * m * m), nb * cin, m, at);
+      gather_mode(gs, dout + static_cast<long long>(b0) * cout * (4 * m * m), nb * cout, m, at);
+      __syncthreads();
+    }
+    auto value = [&](const float2* staged, const float* from, int i) {
+      if (STAGED) return staged[i];
+      const float* src = from + static_cast<long long>(i) * (4 * m * m) + at;
+      return make_float2(src[0], src[m]);
+    };
     for (int t = threadIdx.x; t < cin * cout; t += blockDim.x) {
       const int o = t % cout, i = t / cout;
       float re = b0 ? dwre[wbase + t] : 0.f, im = b0 ? dwim[wbase + t] : 0.f;
       for (int b = 0; b < nb; ++b) {
-        const float2 yv = ys[b * cin + i], gv = gs[b * cout + o];
+        const float2 yv = value(ys, y, b * cin + i), gv = value(gs, dout, b * cout + o);
         const float a = yv.x, c = yv.y, gr = gv.x, gi = gv.y;
         re += __fmaf_rn(a, gr, __fmul_rn(c, gi));
         im += __fmaf_rn(a, gi, -__fmul_rn(c, gr));
@@ -626,9 +641,10 @@ cudaError_t launch_mode_mix(const float* x, const void* wre, const void* wim, fl
                             int n_in, int n_out, int m, cudaStream_t stream) {
   const long long len = ADJOINT ? n_in : n_out;
   const MixStage st = mix_stage(n_in, static_cast<long long>(n_in) * n_out / len * (len + 2), B);
-  const cudaError_t e = allow_smem(mode_mix_kernel<ADJOINT>);
+  auto kernel = st.samples ? mode_mix_kernel<ADJOINT, true> : mode_mix_kernel<ADJOINT, false>;
+  const cudaError_t e = allow_smem(kernel);
   if (e != cudaSuccess) return e;
-  mode_mix_kernel<ADJOINT><<<2 * m * m, 256, st.bytes, stream>>>(
+  kernel<<<2 * m * m, 256, st.bytes, stream>>>(
       x, static_cast<const __nv_bfloat16*>(wre), static_cast<const __nv_bfloat16*>(wim), out,
       static_cast<__nv_bfloat16*>(out_bf), B, n_in, n_out, m, st);
   return cudaGetLastError();
@@ -868,9 +884,9 @@ int pg_fno_mode_mix_backward_bf16(const float* y, const float* dout, const void*
     PG_CUDA(pg::launch_mode_mix<true>(dout, wre, wim, dy, dy_bf16, B, cout, cin, modes, st));
   if (dwre && dwim) {
     const pg::MixStage m = pg::mix_stage(cin + cout, 1LL << 40, B);
-    PG_CUDA(pg::allow_smem(pg::mode_mix_back_weight_kernel));
-    pg::mode_mix_back_weight_kernel<<<2 * modes * modes, 256, m.bytes, st>>>(y, dout, dwre, dwim, B, cin, cout, modes,
-                                                                             m.samples);
+    auto kernel = m.samples ? pg::mode_mix_back_weight_kernel<true> : pg::mode_mix_back_weight_kernel<false>;
+    PG_CUDA(pg::allow_smem(kernel));
+    kernel<<<2 * modes * modes, 256, m.bytes, st>>>(y, dout, dwre, dwim, B, cin, cout, modes, m.samples);
   }
   PG_CUDA(cudaGetLastError());
   return PG_OK;
