@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(RowShape<N, V, COMPS>::MAX_THREADS,
   for (int ph = 0; ph < 2; ++ph) {
     if (ph == 0 ? a.forward : a.inverse) {
       if (ph == 1) conj_all(v);
-      fft_forward<float, N, V>(v, t, buf, 1, tab, sync);
+      fft_forward<N, V>(v, t, buf, 1, tab, sync);
       if (ph == 1) conj_all(v);
     }
     if (ph == 1) continue;
@@ -288,8 +288,8 @@ __device__ __forceinline__ void stage_reservoirs(const IfrkColArgs& a, const flo
 
 // SINGLE: ifrk_sites_batched holds (kernels apart, so that neither path pays the other's registers).
 template <int N, int V, int COMPS, bool SINGLE>
-__global__ void __launch_bounds__(ColShape<float, N, V, COMPS>::MAX_THREADS,
-                                  (ColShape<float, N, V, COMPS>::MIN_BLOCKS + COMPS - 1) / COMPS)
+__global__ void __launch_bounds__(ColShape<N, V, COMPS>::MAX_THREADS,
+                                  (ColShape<N, V, COMPS>::MIN_BLOCKS + COMPS - 1) / COMPS)
     ifrk_col_reg_kernel(float2* __restrict__ psi, const float* __restrict__ n0,
                         float* __restrict__ dn_out, float* __restrict__ n_out,
                         float2* __restrict__ psi_start, float2* __restrict__ psi_new,
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(ColShape<float, N, V, COMPS>::MAX_THREADS,
   for (int ph = 0; ph < 2; ++ph) {
     if (ph == 0 ? a.inverse : a.forward) {
       if (ph == 0) conj_all(v);
-      fft_forward<float, N, V>(v, t, buf, CC, tab, BlockSync{});
+      fft_forward<N, V>(v, t, buf, CC, tab, BlockSync{});
       if (ph == 0) conj_all(v);
     }
     if (ph == 1 || a.mode == 3) continue;
@@ -415,7 +415,7 @@ cudaError_t configure_row() {
 }
 template <int N, int V, int COMPS>
 cudaError_t configure_col() {
-  using S = ColShape<float, N, V, COMPS>;
+  using S = ColShape<N, V, COMPS>;
   const int smem = static_cast<int>(S::MAX_COLS * COMPS * S::SLOTS * sizeof(float2));
   const cudaError_t e = cudaFuncSetAttribute(ifrk_col_reg_kernel<N, V, COMPS, false>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -473,7 +473,7 @@ cudaError_t launch_col(float* psi, const float* n0, float* dn_out, float* n_out,
                        cudaStream_t stream) {
 #define PG_X(N, V)                                                                                     \
   {                                                                                                    \
-    a.cols = col_shape_cols<float, N, V, COMPS>(a.nx, a.members, sm_count);                            \
+    a.cols = col_shape_cols<N, V, COMPS>(a.nx, a.members, sm_count);                            \
     a.log2cols = log2_of(a.cols);                                                                      \
     const dim3 grid(a.nx / a.cols, 1, a.members);                                                      \
     const int threads = a.cols * COMPS * RegFft<N, V>::M;                                              \
@@ -500,8 +500,8 @@ cudaError_t configure_ifrk_reg(int nx, int ny, int comps) {
 
 int ifrk_reg_panels(int nx, int ny, int comps, int members, int sm_count) {
 #define PG_X(N, V)                                                                 \
-  return nx / (comps == 2 ? col_shape_cols<float, N, V, 2>(nx, members, sm_count)  \
-                          : col_shape_cols<float, N, V, 1>(nx, members, sm_count))
+  return nx / (comps == 2 ? col_shape_cols<N, V, 2>(nx, members, sm_count)  \
+                          : col_shape_cols<N, V, 1>(nx, members, sm_count))
   PG_REG_SIZES(ny, PG_X)
 #undef PG_X
   return 0;

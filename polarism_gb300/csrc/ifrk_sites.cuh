@@ -25,9 +25,9 @@ __host__ __device__ inline bool ifrk_sites_batched(const IfrkColArgs& a) {
   return base && ((a.mode == 0 && a.terms <= 5) || (a.mode == 1 && a.terms >= 1 && a.terms <= 5));
 }
 
-// The sites a thread works on: site e = first, first + step, ... below count, at element o of the
-// member's plane and element `slot` of the buffer that holds the field.
-// A panel of C = 2^lc columns of ny rows held as [row][column], dealt over the block.
+// The sites a thread works on, of a panel of C = 2^lc columns of ny rows held as [row][column] and dealt
+// over the block: site e = first, first + step, ... below count, at element o of the member's plane and
+// element `slot` of the panel.
 struct PanelSites {
   int C, lc, nx, x0, total;
   __device__ __forceinline__ int first() const { return static_cast<int>(threadIdx.x); }
@@ -46,9 +46,9 @@ struct PanelSites {
 // in flight; one site at a time, a site's stores would come before the next site's loads,
 // which the compiler may not move above them.  The arithmetic is the generic loop's,
 // expression for expression and in the same order.
-template <typename T, int MODE, int TERMS, int U, typename Sites>
+template <typename T, int MODE, int TERMS, int U>
 __device__ __forceinline__ void ifrk_sites_single(
-    typename C2T<T>::type* buf, const Sites& sites, const IfrkColArgs& a,
+    typename C2T<T>::type* buf, const PanelSites& sites, const IfrkColArgs& a,
     const SplitConst<T>& k, long long mbase, const T* __restrict__ n0,
     T* __restrict__ dn_out, T* __restrict__ n_out, typename C2T<T>::type* __restrict__ psi_start,
     typename C2T<T>::type* __restrict__ psi_new, const T* __restrict__ pm,
@@ -134,9 +134,9 @@ __device__ __forceinline__ void ifrk_sites_single(
 
 // ifrk_sites_single for the launch's mode and term count (ifrk_sites_batched(a) holds); U0 /
 // U1 sites a batch at a stage / the step end.
-template <typename T, int U0, int U1, typename Sites>
+template <typename T, int U0, int U1>
 __device__ __forceinline__ void ifrk_sites_run(
-    typename C2T<T>::type* buf, const Sites& sites, const IfrkColArgs& a,
+    typename C2T<T>::type* buf, const PanelSites& sites, const IfrkColArgs& a,
     const SplitConst<T>& k, long long mbase, const T* n0, T* dn_out, T* n_out,
     typename C2T<T>::type* psi_start, typename C2T<T>::type* psi_new, const T* pm, const T* vm,
     T s0, const PhiloxCellPrefix& prefix) {

@@ -1,5 +1,5 @@
 // Launch shapes and synchronisation shared by the register-resident row and column passes
-// (split_reg.cuh, ifrk_reg.cuh).
+// (split_reg.cu, ifrk_reg.cu).
 #pragma once
 #include <algorithm>
 
@@ -58,29 +58,27 @@ int row_shape_rows(int ny, int members, int sm_count) {
 }
 
 // Column pass: `cols` columns of COMPS components a block.
-template <typename T, int N, int V, int COMPS>
+template <int N, int V, int COMPS>
 struct ColShape {
   static constexpr int M = RegFft<N, V>::M;
   static constexpr int SLOTS = RegFft<N, V>::SLOTS;
-  static constexpr int REGS = sizeof(T) == 4 ? 64 : 128;  // a thread
-  static constexpr int LIMIT = sizeof(T) == 4 ? 1024 : 512;
-  // 64-byte row segments (8 FP32 columns, 4 FP64) while the block stays within LIMIT threads.
+  static constexpr int REGS = 64;  // a thread
+  // 64-byte row segments (8 columns) while the block stays within 1024 threads.
   static constexpr int cap(int want) {
     int c = want;
-    while (c > 1 && c * M * COMPS > LIMIT) c /= 2;
+    while (c > 1 && c * M * COMPS > 1024) c /= 2;
     return c;
   }
-  static constexpr int MAX_COLS = cap(sizeof(T) == 4 ? 8 : 4);
+  static constexpr int MAX_COLS = cap(8);
   static constexpr int MAX_THREADS = MAX_COLS * M * COMPS < 32 ? 32 : MAX_COLS * M * COMPS;
   static constexpr int MIN_BLOCKS = 65536 / (REGS * (MAX_THREADS < 128 ? 128 : MAX_THREADS));
 };
 
-template <typename T, int N, int V, int COMPS>
+template <int N, int V, int COMPS>
 int col_shape_cols(int nx, int members, int sm_count) {
-  using S = ColShape<T, N, V, COMPS>;
+  using S = ColShape<N, V, COMPS>;
   int cols = std::min(S::MAX_COLS, nx);
-  const int least = sizeof(T) == 4 ? 2 : 1;
-  while (cols > least && cols / 2 * S::M * COMPS >= 32 &&
+  while (cols > 2 && cols / 2 * S::M * COMPS >= 32 &&
          5LL * (nx / cols) * members < 4LL * sm_count)
     cols /= 2;
   return cols;

@@ -70,7 +70,7 @@ struct pg_solver {
   void* tw_y = nullptr;
   void* prop = nullptr;       // [table][member][nx + ny] propagator factors
   void* tw4 = nullptr;        // FP32 factors W_1024^{n2 k1} of the 1024-site IFRK column pass
-  void* reg_x = nullptr;      // W_n^{t k} tables of the register-resident passes (split_reg.cuh),
+  void* reg_x = nullptr;      // W_n^{t k} tables of the register-resident passes (split_reg.cu),
   void* reg_y = nullptr;      // rows and columns; null where the size has no such pass
   void* split_consts = nullptr;
   std::map<std::tuple<int, int, int>, cudaGraphExec_t> split_graphs;  // (ordering, len, parity)

@@ -79,7 +79,7 @@ cudaError_t launch_col_pass(T* data, T* res, const T* pump, const T* potential, 
 template <typename T>
 cudaError_t configure_split_kernels(size_t max_smem);
 
-// The FP32 passes on register-resident transforms (split_reg.cuh): axes of 64 to 4096 points.
+// The FP32 passes on register-resident transforms (split_reg.cu): axes of 64 to 4096 points.
 inline bool reg_fft_size(int n) { return n >= 64 && n <= 4096 && (n & (n - 1)) == 0; }
 // Values a thread holds of a transform of n points.  By size alone, so that a member's result does
 // not depend on how many are stepped with it.  Eight to 512 points: a K-outer step of one 256^2 /
