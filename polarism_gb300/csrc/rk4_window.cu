@@ -76,8 +76,8 @@ cudaError_t launch_rk4_window(const float* psi_in, const float* n_in, const floa
   switch (g.wmax) {
 #define PG_WIN_CASE(W)                                                                                  \
   case W:                                                                                               \
-    return launch_rk4_window_##W(psi_in, n_in, pump, psi_out, n_out, consts, scales, step_base,         \
-                                 step_offset, dt, noise, g, err_flag, stream);
+    return launch_window_t<W>(psi_in, n_in, pump, psi_out, n_out, consts, scales, step_base,            \
+                              step_offset, dt, noise, g, err_flag, stream);
     PG_WIN_CASE(256)
     PG_WIN_CASE(320)
     PG_WIN_CASE(512)

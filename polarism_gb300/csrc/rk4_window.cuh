@@ -406,6 +406,8 @@ cudaError_t launch_window_variant(const float* psi_in, const float* n_in, const 
   return cudaGetLastError();
 }
 
+}  // namespace
+
 template <int WMAX>
 cudaError_t launch_window_t(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
                             float* n_out, const RhsConst<float>* consts, const float* scales,
@@ -426,5 +428,4 @@ cudaError_t launch_window_t(const float* psi_in, const float* n_in, const float*
 #undef PG_WIN
 }
 
-}  // namespace
 }  // namespace pg

@@ -3,12 +3,6 @@
 
 namespace pg {
 
-cudaError_t launch_rk4_window_512(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
-                                 float* n_out, const RhsConst<float>* consts, const float* scales,
-                                 const unsigned long long* step_base, int step_offset, float dt, bool noise,
-                                 const WindowGeom& g, int* err_flag, cudaStream_t stream) {
-  return launch_window_t<512>(psi_in, n_in, pump, psi_out, n_out, consts, scales, step_base, step_offset, dt,
-                             noise, g, err_flag, stream);
-}
+template decltype(launch_window_t<512>) launch_window_t<512>;
 
 }  // namespace pg

@@ -42,21 +42,12 @@ cudaError_t launch_rk4_window(const float* psi_in, const float* n_in, const floa
                               float* n_out, const RhsConst<float>* consts, const float* scales,
                               const unsigned long long* step_base, int step_offset, float dt, bool noise,
                               const WindowGeom& g, int* err_flag, cudaStream_t stream);
-cudaError_t launch_rk4_window_256(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
-                              float* n_out, const RhsConst<float>* consts, const float* scales,
-                              const unsigned long long* step_base, int step_offset, float dt, bool noise,
-                              const WindowGeom& g, int* err_flag, cudaStream_t stream);
-cudaError_t launch_rk4_window_320(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
-                              float* n_out, const RhsConst<float>* consts, const float* scales,
-                              const unsigned long long* step_base, int step_offset, float dt, bool noise,
-                              const WindowGeom& g, int* err_flag, cudaStream_t stream);
-cudaError_t launch_rk4_window_512(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
-                              float* n_out, const RhsConst<float>* consts, const float* scales,
-                              const unsigned long long* step_base, int step_offset, float dt, bool noise,
-                              const WindowGeom& g, int* err_flag, cudaStream_t stream);
-cudaError_t launch_rk4_window_1024(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
-                              float* n_out, const RhsConst<float>* consts, const float* scales,
-                              const unsigned long long* step_base, int step_offset, float dt, bool noise,
-                              const WindowGeom& g, int* err_flag, cudaStream_t stream);
+// The same for one window capacity, instantiated in the rk4_window_<capacity>.cu (one each, to compile in
+// parallel).
+template <int WMAX>
+cudaError_t launch_window_t(const float* psi_in, const float* n_in, const float* pump, float* psi_out,
+                            float* n_out, const RhsConst<float>* consts, const float* scales,
+                            const unsigned long long* step_base, int step_offset, float dt, bool noise,
+                            const WindowGeom& g, int* err_flag, cudaStream_t stream);
 
 }  // namespace pg
