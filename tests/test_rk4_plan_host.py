@@ -71,3 +71,19 @@ def test_more_members_than_a_launch_holds(plan):
     ((256, 256, 1), dict(lasers=2), False, (TILE,))])                        # 8.3; windows 9.6
 def test_choice_follows_what_was_measured(plan, grid, options, noise, kernels):
     assert plan(*grid, noise=noise, **options)[0] in kernels
+
+
+@pytest.mark.parametrize("grid,options,noise,kernel", [
+    # us a step of the kernel named against the one that a coarser estimate took: warps that share the schedulers
+    # unevenly, rows of 1024 sites, tiles by the round, the last wave of the streaming kernel's blocks
+    ((1024, 741, 1), {}, True, WINDOW),                                      # 17.6; full width 20.0
+    ((1024, 208, 4), {}, True, WINDOW),                                      # 18.6; full width 20.0
+    ((4096, 133, 2), dict(potential=2), True, WINDOW),                       # 30.5; streaming 34.1
+    ((163, 736, 7), {}, True, WINDOW),                                       # 20.0; streaming 22.2
+    ((595, 93, 7), {}, True, WINDOW),                                        # 13.0; tiles 14.3
+    ((137, 504, 6), dict(potential=2), True, WINDOW),                        # 23.5; streaming 25.4
+    ((128, 128, 96), dict(potential=2), False, WIDE),                        # 33.0; streaming 37.5
+    ((65, 65, 207), dict(potential=2), True, STREAM),                        # windows 20 % slower
+    ((525, 954, 16), dict(reservoir="double"), False, STREAM)])              # 364; tiles 414
+def test_choice_follows_warps_and_rounds(plan, grid, options, noise, kernel):
+    assert plan(*grid, noise=noise, **options)[0] == kernel
